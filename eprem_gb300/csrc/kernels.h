@@ -17,7 +17,8 @@ struct StreamPlan {
   int mmax;      // register slots per thread (>= M)
   int threads;   // threads per CTA
   int cluster;   // CTAs per (stream, energy) slab
-  int reg_coef;  // coefficients in registers (1), shared memory (0); 2: stream2.cu
+  int reg_coef;  // coefficients in registers (1), shared memory (0); 2: stream2.cu;
+                 // 3: stream64.cu
   int packed;    // stream2.cu: fp32x2 arithmetic on pairs of mu cells
   int filled;    // stream2.cu: M fills the bin, m0 = M/2 (guards known at compile time)
   int npt;       // stream2.cu: list nodes per thread
@@ -29,6 +30,10 @@ int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, Strea
 int launch_stream(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                   uint64_t *launches);
 int launch_seed_check(const RunView &r, cudaStream_t st, uint64_t *launches);
+// stream64.cu -- FP64 streaming in three operations per cell (plan.reg_coef == 3)
+bool stream64_shape(int N, int M, int m0, StreamPlan *plan);
+int launch_stream64(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
+                    uint64_t *launches);
 // stream2.cu -- FP32 streaming, two list nodes per thread (plan.reg_coef == 2)
 // shape: 0 automatic, k >= 1 the k-th CTA shape of M's bin (stream2_shape_count)
 // mirror: 0, or the mirrored kind (1, 2: StreamPlan::mirror), which needs filled and bc

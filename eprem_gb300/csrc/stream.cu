@@ -13,8 +13,10 @@
 //   * the isotropisation mean over mu is a register sum in the owning thread.
 // The upwind coefficients mult*del_fac are fixed for the slab and held in
 // shared memory (the FP64 form is bound by the FP64 pipe, next to which
-// shared-memory loads cost nothing).  This is the plain FP64 form's kernel;
-// the FP32 form streams with stream2.cu.
+// shared-memory loads cost nothing).  This is the plain FP64 form's kernel for
+// streams too long for stream64.cu, which takes three FP64 operations per cell
+// and sub-cycle where this one takes four but twice the shared memory; the
+// FP32 form streams with stream2.cu.
 // seedPopulationCheck (src/energeticParticlesBoundary.c:28-59) is applied as
 // the slab is loaded; thinned-out nodes receive their reference node's values
 // on write-back, as the reference's shellRef copy does (:2448-2455).
@@ -271,8 +273,9 @@ static int threads_for(int mmax) {
 // on the sub-cycle loop, 7 from shared memory; both need the seed boundary)
 // -- the automatic kind is the first of 7, 5, 4, 3 that fits; shape 0 lets
 // plan_stream2 choose the CTA shape from N, k >= 1 names the k-th shape of
-// the mu bin.  The FP64 form has one shape (k_stream, coefficients in shared
-// memory); variants 1 and 2 name it there.
+// the mu bin.  The FP64 form has one kernel per stream length (stream64.cu, or
+// k_stream where a cluster of that one cannot hold the stream); variants 1 and
+// 2 name it there.
 int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, StreamPlan *plan) {
   if (precision == EPREM_FP32) {
     const int kind = variant % 8, shape = variant / 8;
@@ -290,6 +293,7 @@ int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, Strea
     return EPREM_GPU_ERR_ARG;
   }
   if (variant > 2) return EPREM_GPU_ERR_ARG;
+  if (stream64_shape(N, M, m0, plan)) return 0;
   int mmax = 0;
   for (int b : kStreamBins)
     if (M <= b) { mmax = b; break; }
@@ -344,6 +348,7 @@ int launch_stream(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t
                   uint64_t *launches) {
   if (plan.reg_coef == 2) return launch_stream2(r, plan, m0, st, launches);
   if (r.precision != EPREM_FP64) return EPREM_GPU_ERR_ARG;
+  if (plan.reg_coef == 3) return launch_stream64(r, plan, m0, st, launches);
   const cudaError_t err = dispatch_mmax<double, false>(r, plan, m0, st);
   *launches += 1;
   return err == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
