@@ -49,6 +49,7 @@ struct EnergyConsts {
   float dvi32;           // vgrid_i[e+1] - vgrid_i[e-1] (0 at the ends), from FP64
   int seed_k;            // FP32 streaming seeds are held as seed * 2^seed_k, so that
                          // the energy-only factor of sepSeedFunction is near 1
+  double two_vi;         // 2 / vgrid (the focusing speed's factor of DuPar)
   double drift_factor;   // (1/om1) p v / 3 of driftVelocity (src/energeticParticles.c:
                          // 210-246), p = exp(lnpmin + E dlnp); 0 without drift
 };
@@ -65,6 +66,15 @@ struct NodeCoef32 {
   // value relative to a row's exponent without losing the fraction
   float bc0, bc1;
   int kbc0, kbc1;
+};
+
+// The same for the FP64 kernel (node64.cu), in double; step_f, step_c: the
+// sub-cycle's dt over dmu / dlnp.
+struct NodeCoef64 {
+  int ok, ns_f, ns_c, pad0;
+  double dlnbds, dupar, b, step_f;
+  double cool, dlnb, dlnn, step_c;
+  double bc0, bc1;  // ln seed at the first and last energy
 };
 
 struct RunView {
@@ -85,6 +95,7 @@ struct RunView {
   double *seed_radial;     // [S*N]   pow(r/normRadius, -beta)
   double *mfp_node;        // [S*N]   pow(r*rScale, a) or pow(BsAu/B, b)
   NodeCoef32 *coef32;      // [S*N]   FP32 form only
+  NodeCoef64 *coef64;      // [S*N]   FP64 form with Euler or RK3 operators only
   float4 *scoef;           // [S][E][N] FP32 streaming coefficients (stream2.cu)
   DevStatus *status;
   // parameters

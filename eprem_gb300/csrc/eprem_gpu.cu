@@ -150,8 +150,14 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
                       params->adiabatic_change_alg == 1;
   const bool bc = params->use_ep_boundary > 0 && params->use_boundary_function > 0;
   int prc = plan_stream(dims->precision, N, M, m0, params->stream_variant, bc, &r->splan);
-  if (!prc) prc = fast32 ? plan_node32(E, M, &r->nplan) : plan_node(dims->precision, E, M, &r->nplan);
+  const bool fast64 = dims->precision == EPREM_FP64 && params->adiabatic_focus_alg <= 2 &&
+                      params->adiabatic_change_alg <= 2;
+  if (!prc)
+    prc = fast32   ? plan_node32(E, M, &r->nplan)
+          : fast64 ? plan_node64(E, M, params->adiabatic_focus_alg, &r->nplan)
+                   : plan_node(dims->precision, E, M, &r->nplan);
   r->nplan.fast32 = fast32 ? 1 : 0;
+  r->nplan.fast64 = fast64 ? 1 : 0;
   if (prc) {
     delete r;
     return fail(EPREM_GPU_ERR_ARG, "sizes exceed the supported kernel shapes "
@@ -177,6 +183,7 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
   if (e == cudaSuccess) e = dalloc(&r->d_mugrid, (size_t)M);
   if (e == cudaSuccess) e = dalloc(&r->d_mugrid32, (size_t)M);
   if (e == cudaSuccess && fast32) e = dalloc(&r->d_coef32, SN);
+  if (e == cudaSuccess && fast64) e = dalloc(&r->d_coef64, SN);
   // FP32 streaming coefficients (any FP32 run may be tuned to stream2.cu)
   if (e == cudaSuccess && dims->precision == EPREM_FP32 && params->use_parallel_diffusion > 0)
     e = dalloc(&r->d_scoef, SN * (size_t)dims->num_energies);
@@ -209,6 +216,7 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
     ec[i].rig_lamo = grids->rigidity[i] * p.lamo;
     ec[i].seed_power = pow((grids->egrid[i] / normE1), -p.bf_gamma);
     ec[i].seed_exp = exp(-(grids->egrid[i] / normE0));
+    ec[i].two_vi = 2.0 / grids->vgrid[i];
     ec[i].v32 = (float)grids->vgrid[i];
     ec[i].vi32 = (float)grids->vgrid_i[i];
     ec[i].dvi32 = (i >= 1 && i + 1 < E)
@@ -248,6 +256,7 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
   v.mugrid = r->d_mugrid;
   v.mugrid32 = r->d_mugrid32;
   v.coef32 = r->d_coef32;
+  v.coef64 = r->d_coef64;
   v.scoef = r->d_scoef;
   v.ec = r->d_ec;
   v.list = r->d_list;
@@ -308,6 +317,7 @@ extern "C" int eprem_gpu_destroy(eprem_gpu_run *r) {
   cudaFree(r->d_surr_counts);
   cudaFree(r->d_reject);
   cudaFree(r->d_coef32);
+  cudaFree(r->d_coef64);
   cudaFree(r->d_scoef);
   cudaFree(r->d_ec);
   cudaFree(r->d_list);
@@ -538,6 +548,7 @@ static RunView stream_range_view(const eprem_gpu_run *r, int s0, int s1) {
   u.seed_radial = v.seed_radial + n0;
   u.mfp_node = v.mfp_node + n0;
   if (u.coef32) u.coef32 = v.coef32 + n0;
+  if (u.coef64) u.coef64 = v.coef64 + n0;
   if (u.scoef) u.scoef = v.scoef + (size_t)s0 * v.E * v.N;
   return u;
 }
@@ -551,7 +562,7 @@ int eprem::ep_begin(eprem_gpu_run *r, const RunView &v) {
   int rc = timed(r, EPREM_KERNEL_GEOMETRY, [&] {
     return launch_geometry(v, r->stream, r->norm_radius, r->neg_beta, p.mfp_type,
                            p.mfp_type == 2 ? p.mfp_b_power : p.mfp_radial_power, p.mhd_bs_au,
-                           &r->launches);
+                           &r->launches, true);
   });
   if (rc) return cuda_fail(cudaGetLastError(), "geometry launch");
   if (v.use_stream && r->splan.reg_coef == 2) {
@@ -603,8 +614,9 @@ int eprem::ep_node_phase(eprem_gpu_run *r, const RunView &v) {
     if (rc) return rc == EPREM_GPU_ERR_CUDA ? cuda_fail(cudaGetLastError(), "split node phase") : rc;
   } else if (v.use_focus || v.use_change) {
     rc = timed(r, EPREM_KERNEL_NODE, [&] {
-      return r->nplan.fast32 ? launch_node32(v, r->nplan, r->stream, &r->launches)
-                             : launch_node(v, r->nplan, r->stream, &r->launches);
+      return r->nplan.fast32   ? launch_node32(v, r->nplan, r->stream, &r->launches)
+             : r->nplan.fast64 ? launch_node64(v, r->nplan, r->stream, &r->launches)
+                               : launch_node(v, r->nplan, r->stream, &r->launches);
     });
     if (rc) return cuda_fail(cudaGetLastError(), "focusing/change launch");
   }

@@ -9,8 +9,11 @@
 //   * min_tau over nodes >= 1 (src/energeticParticles.c:149-156);
 //   * GetStreamList + FindSegmentLengths (src/energeticParticles.c:2150-2234,
 //     :2496-2601): thinned list, 1/ds of list segments, dsMin per stream.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
+#include "noderates.cuh"
 
 namespace eprem {
 
@@ -20,59 +23,89 @@ __device__ __forceinline__ double dist3(double dx, double dy, double dz) {
   return sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
 }
 
+// One thread per node.  RATES: the FP64 form's focusing / change coefficients
+// too (NodeCoef64); the FP32 form forms its own (node32.cu).
+template <bool RATES>
 __global__ void k_node_prep(RunView r, double norm_radius, double neg_beta, int mfp_type,
                             double mfp_power, double bs_au) {
   const size_t SN = (size_t)r.S * r.N;
-  for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < SN;
-       g += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(g % r.N);
-    const double rs = r.r_scale;
-    const double *rx = node_field(r, EPREM_NODE_RX), *ry = node_field(r, EPREM_NODE_RY),
-                 *rz = node_field(r, EPREM_NODE_RZ), *bmag = node_field(r, EPREM_NODE_BMAG);
-    // __dmul_rn keeps the scaled coordinates out of fused multiply-adds with
-    // the differences below (the reference scales, then subtracts).
-    double x = __dmul_rn(rx[g], rs), y = __dmul_rn(ry[g], rs), z = __dmul_rn(rz[g], rs);
-    double ds, bminus, bplus;
-    if (k == 0) {
-      double px = __dmul_rn(rx[g + 1], rs), py = __dmul_rn(ry[g + 1], rs),
-             pz = __dmul_rn(rz[g + 1], rs);
-      ds = dist3(px - x, py - y, pz - z);
-      bminus = bmag[g];
-      bplus = bmag[g + 1];
-    } else if (k == r.N - 1) {
-      double mx = __dmul_rn(rx[g - 1], rs), my = __dmul_rn(ry[g - 1], rs),
-             mz = __dmul_rn(rz[g - 1], rs);
-      ds = dist3(x - mx, y - my, z - mz);
-      bminus = bmag[g - 1];
-      bplus = bmag[g];
-    } else {
-      double px = __dmul_rn(rx[g + 1], rs), py = __dmul_rn(ry[g + 1], rs),
-             pz = __dmul_rn(rz[g + 1], rs);
-      double mx = __dmul_rn(rx[g - 1], rs), my = __dmul_rn(ry[g - 1], rs),
-             mz = __dmul_rn(rz[g - 1], rs);
-      double dsp = dist3(px - x, py - y, pz - z);
-      double dsm = dist3(x - mx, y - my, z - mz);
-      ds = 0.5 * (dsp + dsm);
-      bminus = bmag[g - 1];
-      bplus = bmag[g + 1];
-    }
-    node_field(r, EPREM_NODE_DS)[g] = ds;
-    node_field(r, EPREM_NODE_BMAG_MINUS)[g] = bminus;
-    node_field(r, EPREM_NODE_BMAG_PLUS)[g] = bplus;
-    const double rmag = node_field(r, EPREM_NODE_RMAG)[g];
-    // radialTerm of sepSeedFunction (src/energeticParticlesBoundary.c:100)
-    r.seed_radial[g] = pow(rmag / norm_radius, neg_beta);
-    // pow factor of meanFreePathR / meanFreePathB (src/meanFreePath.c:13-27)
-    double mf = (mfp_type == 2) ? pow(bs_au / bmag[g], mfp_power) : pow(rmag * rs, mfp_power);
-    r.mfp_node[g] = mf;
-    if (k >= 1) {
-      double tmin = DBL_MAX;
-      for (int e = 0; e < r.E; e++) {
-        double tau = r.ec[e].rig_lamo * mf * r.ec[e].vgrid_i;
-        if (tau < tmin) tmin = tau;
+  for (size_t g0 = blockIdx.x * (size_t)blockDim.x; g0 < SN; g0 += (size_t)gridDim.x * blockDim.x) {
+    const size_t g = g0 + threadIdx.x;
+    int ns_f = 0, ns_c = 0;
+    if (g < SN) {
+      const int k = (int)(g % r.N);
+      const double rs = r.r_scale;
+      const double *rx = node_field(r, EPREM_NODE_RX), *ry = node_field(r, EPREM_NODE_RY),
+                   *rz = node_field(r, EPREM_NODE_RZ), *bmag = node_field(r, EPREM_NODE_BMAG);
+      // __dmul_rn keeps the scaled coordinates out of fused multiply-adds with
+      // the differences below (the reference scales, then subtracts).
+      double x = __dmul_rn(rx[g], rs), y = __dmul_rn(ry[g], rs), z = __dmul_rn(rz[g], rs);
+      double ds, bminus, bplus;
+      if (k == 0) {
+        double px = __dmul_rn(rx[g + 1], rs), py = __dmul_rn(ry[g + 1], rs),
+               pz = __dmul_rn(rz[g + 1], rs);
+        ds = dist3(px - x, py - y, pz - z);
+        bminus = bmag[g];
+        bplus = bmag[g + 1];
+      } else if (k == r.N - 1) {
+        double mx = __dmul_rn(rx[g - 1], rs), my = __dmul_rn(ry[g - 1], rs),
+               mz = __dmul_rn(rz[g - 1], rs);
+        ds = dist3(x - mx, y - my, z - mz);
+        bminus = bmag[g - 1];
+        bplus = bmag[g];
+      } else {
+        double px = __dmul_rn(rx[g + 1], rs), py = __dmul_rn(ry[g + 1], rs),
+               pz = __dmul_rn(rz[g + 1], rs);
+        double mx = __dmul_rn(rx[g - 1], rs), my = __dmul_rn(ry[g - 1], rs),
+               mz = __dmul_rn(rz[g - 1], rs);
+        double dsp = dist3(px - x, py - y, pz - z);
+        double dsm = dist3(x - mx, y - my, z - mz);
+        ds = 0.5 * (dsp + dsm);
+        bminus = bmag[g - 1];
+        bplus = bmag[g + 1];
       }
-      atomic_min_pos(&r.status->min_tau_bits, tmin);
+      node_field(r, EPREM_NODE_DS)[g] = ds;
+      node_field(r, EPREM_NODE_BMAG_MINUS)[g] = bminus;
+      node_field(r, EPREM_NODE_BMAG_PLUS)[g] = bplus;
+      const double rmag = node_field(r, EPREM_NODE_RMAG)[g];
+      // radialTerm of sepSeedFunction (src/energeticParticlesBoundary.c:100)
+      const double radial = pow(rmag / norm_radius, neg_beta);
+      r.seed_radial[g] = radial;
+      // pow factor of meanFreePathR / meanFreePathB (src/meanFreePath.c:13-27)
+      double mf = (mfp_type == 2) ? pow(bs_au / bmag[g], mfp_power) : pow(rmag * rs, mfp_power);
+      r.mfp_node[g] = mf;
+      if (k >= 1) {
+        double tmin = DBL_MAX;
+        for (int e = 0; e < r.E; e++) {
+          double tau = r.ec[e].rig_lamo * mf * r.ec[e].vgrid_i;
+          if (tau < tmin) tmin = tau;
+        }
+        atomic_min_pos(&r.status->min_tau_bits, tmin);
+      }
+      if constexpr (RATES) {
+        const rates::NodeRates o = rates::node_rates(r, g, k, ds, bplus, bminus);
+        ns_f = o.ns_f;
+        ns_c = o.ns_c;
+        NodeCoef64 c{};
+        c.ok = k != 0;
+        c.ns_f = ns_f;
+        c.ns_c = ns_c;
+        c.dlnbds = o.dlnbds;
+        c.dupar = o.dupar;
+        c.b = o.b;
+        c.step_f = (r.dt / ns_f) / r.dmu;
+        c.cool = o.cool;
+        c.dlnb = o.dlnb;
+        c.dlnn = o.dlnn;
+        c.step_c = (r.dt / ns_c) / r.dlnp;
+        if (r.use_change) {
+          c.bc0 = log(seed_value(r, r.ec[0], radial));
+          c.bc1 = log(seed_value(r, r.ec[r.E - 1], radial));
+        }
+        r.coef64[g] = c;
+      }
     }
+    if constexpr (RATES) rates::count_nodes(r, ns_f, ns_c);
   }
 }
 
@@ -152,11 +185,16 @@ __global__ void k_stream_list(RunView r) {
 }
 
 int launch_geometry(const RunView &r, cudaStream_t st, double norm_radius, double neg_beta,
-                    int mfp_type, double mfp_power, double bs_au, uint64_t *launches) {
+                    int mfp_type, double mfp_power, double bs_au, uint64_t *launches,
+                    bool node_rates) {
   const size_t SN = (size_t)r.S * r.N;
-  int blocks = (int)((SN + 255) / 256);
-  if (blocks > 152 * 32) blocks = 152 * 32;
-  k_node_prep<<<blocks, 256, 0, st>>>(r, norm_radius, neg_beta, mfp_type, mfp_power, bs_au);
+  // 64 threads a CTA: FP64 latency bounds a node's chain, and a small run has
+  // no more than a warp or two per SM
+  const int blocks = (int)std::min<size_t>((SN + 63) / 64, 152 * 64);
+  if (node_rates && r.coef64)
+    k_node_prep<true><<<blocks, 64, 0, st>>>(r, norm_radius, neg_beta, mfp_type, mfp_power, bs_au);
+  else
+    k_node_prep<false><<<blocks, 64, 0, st>>>(r, norm_radius, neg_beta, mfp_type, mfp_power, bs_au);
   size_t smem = (size_t)r.N * (3 * sizeof(double) + sizeof(int));
   // per launch: runs of different sizes share the kernel's attribute
   if (cudaFuncSetAttribute(k_stream_list, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -8,8 +8,11 @@
 namespace eprem {
 
 // geometry.cu
+// node_rates: also the node coefficients and sub-cycle counts (added to the
+// statistics) of the FP64 form's node64.cu, once per updateEnergeticParticles
 int launch_geometry(const RunView &r, cudaStream_t st, double norm_radius, double neg_beta,
-                    int mfp_type, double mfp_power, double bs_au, uint64_t *launches);
+                    int mfp_type, double mfp_power, double bs_au, uint64_t *launches,
+                    bool node_rates = false);
 int setup_geometry_attrs(int N);
 
 // stream.cu -- DiffuseStreamData (+ seedPopulationCheck)
@@ -64,9 +67,13 @@ struct NodePlan {
   int nodes;       // nodes per CTA
   size_t smem;     // dynamic shared memory bytes
   int fast32;      // FP32 form with Euler operators: node32.cu
+  int fast64;      // FP64 form with Euler or RK3 operators: node64.cu
 };
 int plan_node(int precision, int E, int M, NodePlan *plan);
 int launch_node(const RunView &r, const NodePlan &plan, cudaStream_t st, uint64_t *launches);
+// node64.cu -- FP64-form focusing + change (Euler and RK3 operators)
+int plan_node64(int E, int M, int focus_alg, NodePlan *plan);
+int launch_node64(const RunView &r, const NodePlan &plan, cudaStream_t st, uint64_t *launches);
 // node32.cu -- FP32-form focusing + change (Euler operators)
 int plan_node32(int E, int M, NodePlan *plan);
 int launch_node32(const RunView &r, const NodePlan &plan, cudaStream_t st, uint64_t *launches);

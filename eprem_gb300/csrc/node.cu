@@ -1,6 +1,7 @@
 // node.cu -- adiabatic focusing and adiabatic change per node (K23).
 //
-// Restates, for every node but the innermost of each stream (innerComputeShell,
+// The FP32 form with third-order operators and, in either form, WENO3 (the other
+// algorithms: node32.cu, node64.cu).  Restates, for every node but the innermost of each stream (innerComputeShell,
 // src/mpiInit.c:105-109):
 //   AdiabaticFocusing  (src/energeticParticles.c:1537-1803) -- advection in mu
 //     along each energy row, sub-cycled to the node's CFL limit;

@@ -44,6 +44,7 @@ struct eprem_gpu_run {
   double *d_nodes = nullptr, *d_mugrid = nullptr;
   float *d_mugrid32 = nullptr;
   eprem::NodeCoef32 *d_coef32 = nullptr;
+  eprem::NodeCoef64 *d_coef64 = nullptr;
   float4 *d_scoef = nullptr;
   eprem::EnergyConsts *d_ec = nullptr;
   int *d_list = nullptr, *d_list_size = nullptr;
