@@ -60,13 +60,15 @@ int tune_stream(eprem_gpu_run *r, int *chosen) {
   StreamPlan best_plan{};
   uint64_t dummy = 0;
   std::vector<int> variants;
-  for (int shape = 1; shape <= stream2_shape_count(r->dims.num_mu); ++shape)
-    for (int kind : kTuneKinds) variants.push_back(kind + 8 * shape);
+  const int M = r->dims.num_mu, old = stream2_shape_count(M), wide = stream2m_width_count(M);
+  for (int shape = 1; shape <= old + wide; ++shape)
+    for (int kind : kTuneKinds)  // the mirrored kernel's widths: kinds 6, 7, or after the bin's shapes
+      if (kind >= 6 ? r->mirror_ok && shape <= wide : true) variants.push_back(kind + 8 * shape);
   for (int variant : variants) {
     if (e != cudaSuccess) break;
     StreamPlan pl{};
     if (plan_stream(EPREM_FP32, r->dims.num_nodes, r->dims.num_mu, r->m0, variant,
-                    r->v.use_bc != 0, &pl))
+                    r->v.use_bc != 0, r->mirror_ok, r->slabs(), &pl))
       continue;
     if (launch_stream(v, pl, r->m0, r->stream, &dummy)) {  // warm-up
       e = cudaGetLastError();
@@ -114,11 +116,14 @@ extern "C" int eprem_gpu_plan_stream(int num_nodes, int num_mu, int m0, int prec
   if (!out || num_nodes < 3 || num_mu < 2 || num_mu > 64 || m0 < 0 || m0 > num_mu)
     return fail(EPREM_GPU_ERR_ARG, "bad sizes");
   StreamPlan p{};
-  if (plan_stream(precision, num_nodes, num_mu, m0, variant, seed_boundary != 0, &p))
+  // (a run with few slabs may take a narrower shape)
+  if (plan_stream(precision, num_nodes, num_mu, m0, variant, seed_boundary != 0,
+                  seed_boundary != 0, 1 << 20, &p))
     return fail(EPREM_GPU_ERR_ARG, "no streaming kernel fits these sizes");
   const bool s2 = p.reg_coef == 2;
-  out[0] = !s2 ? 0 : p.mirror ? 5 + p.mirror : !p.packed ? 3 : p.filled ? 5 : 4;
-  out[1] = p.mmax;
+  const bool own = p.mirror && (num_mu == 20 || num_mu == 40);
+  out[0] = !s2 ? 0 : own ? 7 : !p.packed ? 3 : p.filled ? 5 : 4;
+  out[1] = p.mirror && !own ? stream2_bin(num_mu) : p.mmax;
   out[2] = p.threads;
   out[3] = s2 ? p.npt : 1;
   out[4] = p.cluster;
@@ -135,7 +140,7 @@ extern "C" const char *eprem_gpu_stream_kernel(eprem_gpu_run *r) {
              p.mmax, p.cluster);
   else
     snprintf(buf, sizeof(buf), "%s<%d,%d,%d> cluster %d",
-             p.mirror ? "k_stream2_mirror" : p.packed ? "k_stream2_pairs" : "k_stream2", p.mmax,
+             p.mirror ? "k_stream2m" : p.packed ? "k_stream2_pairs" : "k_stream2", p.mmax,
              p.threads, p.npt, p.cluster);
   r->skernel = buf;
   return r->skernel.c_str();
@@ -145,7 +150,7 @@ extern "C" int eprem_gpu_set_stream_variant(eprem_gpu_run *r, int variant) {
   if (!r) return fail(EPREM_GPU_ERR_ARG, "null run");
   StreamPlan pl{};
   if (plan_stream(r->dims.precision, r->dims.num_nodes, r->dims.num_mu, r->m0, variant,
-                  r->v.use_bc != 0, &pl))
+                  r->v.use_bc != 0, r->mirror_ok, r->slabs(), &pl))
     return fail(EPREM_GPU_ERR_ARG, "streaming variant does not fit this run's sizes");
   r->splan = pl;
   r->params.stream_variant = variant;
@@ -173,6 +178,7 @@ struct eprem_gpu_ensemble {
   int chains = -1;  // < 0 lock-step with merged streaming; 0 one branch per run; k serial chains
   // lock-step: the slab lists of the merged streaming launches
   std::vector<int4 *> d_items;
+  std::vector<RunView *> d_views;  // and their runs' views
 };
 
 static void ensemble_drop_graph(eprem_gpu_ensemble *e) {
@@ -181,7 +187,9 @@ static void ensemble_drop_graph(eprem_gpu_ensemble *e) {
   e->exec = nullptr;
   e->graph = nullptr;
   for (int4 *p : e->d_items) cudaFree(p);
+  for (RunView *p : e->d_views) cudaFree(p);
   e->d_items.clear();
+  e->d_views.clear();
 }
 
 extern "C" int eprem_gpu_ensemble_destroy(eprem_gpu_ensemble *e) {
@@ -261,7 +269,7 @@ extern "C" int eprem_gpu_ensemble_autotune(eprem_gpu_ensemble *e, int *chosen_va
     eprem_gpu_run *r = e->runs[i];
     StreamPlan key{};
     plan_stream(r->dims.precision, r->dims.num_nodes, r->dims.num_mu, r->m0, 0,
-                r->v.use_bc != 0, &key);
+                r->v.use_bc != 0, r->mirror_ok, r->slabs(), &key);
     const std::vector<int> k = {r->dims.precision, key.mmax, key.cluster, key.threads,
                                 r->dims.num_mu, r->m0};
     int variant = -1;
@@ -329,9 +337,22 @@ static int ensemble_capture_lockstep(eprem_gpu_ensemble *e) {
   }
   std::vector<S2Group> groups;
   std::vector<int> solo;
+  // runs of one size share a launch: the automatic shape is chosen for all
+  // their slabs (a slab's values do not depend on the shape)
+  auto merged_plan = [&](eprem_gpu_run *r) {
+    StreamPlan pl = r->splan;
+    if (!pl.mirror || r->params.stream_variant / 8) return pl;
+    long long slabs = 0;
+    for (eprem_gpu_run *o : e->runs)
+      if (o->splan.mirror && !(o->params.stream_variant / 8) && o->dims.num_mu == r->dims.num_mu &&
+          o->dims.num_nodes == r->dims.num_nodes)
+        slabs += o->slabs();
+    plan_stream2m(r->dims.num_nodes, r->dims.num_mu, r->m0, true, 0, slabs, &pl);
+    return pl;
+  };
   for (int i = 0; i < n; i++) {
     eprem_gpu_run *r = e->runs[i];
-    const StreamPlan &pl = r->splan;
+    const StreamPlan pl = merged_plan(r);
     if (!r->v.use_stream || pl.reg_coef != 2 || !pl.packed) {
       solo.push_back(i);
       continue;
@@ -371,6 +392,11 @@ static int ensemble_capture_lockstep(eprem_gpu_ensemble *e) {
     e->d_items.push_back(d);
     CK(cudaMemcpy(d, flat.data(), flat.size() * sizeof(int4), cudaMemcpyHostToDevice));
     n_items[gi] = (int)flat.size();
+    RunView *dv = nullptr;
+    CK(cudaMalloc(&dv, sizeof(RunView) * groups[gi].runs.size()));
+    e->d_views.push_back(dv);
+    CK(cudaMemcpy(dv, views[gi].v, sizeof(RunView) * groups[gi].runs.size(),
+                  cudaMemcpyHostToDevice));
   }
   // node phases: runs of one mu count in the plain form, focusing and change
   // both on, in two launches per sub-step over all their (run, block) items
@@ -436,7 +462,8 @@ static int ensemble_capture_lockstep(eprem_gpu_ensemble *e) {
   }
   for (int step = 0; step < nsub && !rc && err == cudaSuccess; step++) {
     for (size_t gi = 0; gi < groups.size() && !rc; gi++)
-      if (launch_stream2_multi(groups[gi].plan, views[gi], e->d_items[gi], n_items[gi],
+      if (launch_stream2_multi(groups[gi].plan, views[gi], e->d_views[gi], e->d_items[gi],
+                               n_items[gi],
                                e->origin, &e->runs[groups[gi].runs[0]]->launches))
         err = cudaGetLastError();
     for (int i : solo)

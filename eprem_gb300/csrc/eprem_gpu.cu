@@ -149,7 +149,14 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
   const bool fast32 = dims->precision == EPREM_FP32 && params->adiabatic_focus_alg == 1 &&
                       params->adiabatic_change_alg == 1;
   const bool bc = params->use_ep_boundary > 0 && params->use_boundary_function > 0;
-  int prc = plan_stream(dims->precision, N, M, m0, params->stream_variant, bc, &r->splan);
+  // the mirrored streaming kernel takes |mugrid| of a cell from its mirror cell
+  bool even_mu = true;
+  for (int m = 0; m < M; m++)
+    even_mu = even_mu && fabs(grids->mugrid[m] + grids->mugrid[M - 1 - m]) <= 1e-9 &&
+              fabs(grids->mugrid[m] - grids->mugrid[0] - m * grids->dmu) <= 1e-9;
+  r->mirror_ok = bc && even_mu;
+  int prc = plan_stream(dims->precision, N, M, m0, params->stream_variant, bc, r->mirror_ok,
+                        (long long)S * E, &r->splan);
   const bool fast64 = dims->precision == EPREM_FP64 && params->adiabatic_focus_alg <= 2 &&
                       params->adiabatic_change_alg <= 2;
   if (!prc)
@@ -688,15 +695,22 @@ extern "C" int eprem_gpu_update_energetic_particles_host(eprem_gpu_run *r, const
     return rc;
   }
   // Chunks: a short first and last one (1/32 of the streams each: the first
-  // upload and the last download are the copies nothing hides) around six
-  // long ones, whose copies each take less than a neighbour's update.
+  // upload and the last download are the copies nothing hides) around up to
+  // six long ones, whose copies each take less than a neighbour's update.  A
+  // chunk keeps at least kChunkSlabs (stream, energy) slabs, a run with fewer
+  // than twice that goes in one piece: a launch over few slabs leaves SMs idle
+  // while its longest ones finish, which costs more than the copies (54 streams
+  // x 632 x 38 x 22, 2052 slabs, a step of 30 sub-steps: 79 ms of streaming in
+  // eight chunks, 30 in one, and 5 ms of copies).
+  constexpr long long kChunkSlabs = 152 * 8;
   std::vector<int> bounds{0};
-  const int edge = S >= 64 ? (S + 31) / 32 : (S >= 8 ? 1 : 0);
+  const int pieces = (int)std::min<long long>(6, r->slabs() / kChunkSlabs);
+  const int edge = pieces < 2 ? 0 : S >= 64 ? (S + 31) / 32 : (S >= 8 ? 1 : 0);
   if (edge) {
     const int mid = S - 2 * edge;
     bounds.push_back(edge);
-    for (int i = 1; i <= 6; i++) {
-      const int b = edge + (int)((long long)mid * i / 6);
+    for (int i = 1; i <= pieces; i++) {
+      const int b = edge + (int)((long long)mid * i / pieces);
       if (b > bounds.back()) bounds.push_back(b);
     }
   }

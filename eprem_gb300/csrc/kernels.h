@@ -25,11 +25,12 @@ struct StreamPlan {
   int packed;    // stream2.cu: fp32x2 arithmetic on pairs of mu cells
   int filled;    // stream2.cu: M fills the bin, m0 = M/2 (guards known at compile time)
   int npt;       // stream2.cu: list nodes per thread
-  int mirror;    // stream2.cu: mu < 0 half in mirror order, one coefficient per two cells
-                 // (1 formed on the sub-cycle loop, 2 from shared memory)
+  int mirror;    // stream2m.cu (mmax is M itself there)
 };
-// bc: the run has the seed boundary (the mirrored kinds need it)
-int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, StreamPlan *plan);
+// bc: the run has the seed boundary (the mirrored kernel needs it); mirror_ok:
+// and a uniform symmetric mu grid; slabs: (stream, energy) slabs of a launch
+int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool mirror_ok,
+                long long slabs, StreamPlan *plan);
 int launch_stream(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                   uint64_t *launches);
 int launch_seed_check(const RunView &r, cudaStream_t st, uint64_t *launches);
@@ -37,25 +38,35 @@ int launch_seed_check(const RunView &r, cudaStream_t st, uint64_t *launches);
 bool stream64_shape(int N, int M, int m0, StreamPlan *plan);
 int launch_stream64(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                     uint64_t *launches);
-// stream2.cu -- FP32 streaming, two list nodes per thread (plan.reg_coef == 2)
+// stream2.cu -- FP32 streaming, several list nodes per thread (plan.reg_coef == 2)
 // shape: 0 automatic, k >= 1 the k-th CTA shape of M's bin (stream2_shape_count)
-// mirror: 0, or the mirrored kind (1, 2: StreamPlan::mirror), which needs filled and bc
-int plan_stream2(int N, int M, int m0, bool packed, bool filled, int mirror, bool bc, int shape,
-                 StreamPlan *plan);
+int plan_stream2(int N, int M, int m0, bool packed, bool filled, int shape, StreamPlan *plan);
+bool stream2_filled(int M, int m0);  // M fills its bin in halves of equal length
+int stream2_bin(int M);              // the bin a plan of M is reported under
 int stream2_shape_count(int M);
 // The packed kinds over the slabs of several runs of one plan: the runs'
-// views (a kernel parameter) and items[i] = (run index, stream, energy, 0)
+// views (a kernel parameter; also in device memory for the mirrored kernel)
+// and items[i] = (run index, stream, energy, 0)
 constexpr int kMultiRuns = 64;
 struct MultiRunViews {
   RunView v[kMultiRuns];
   int m0[kMultiRuns];
 };
-int launch_stream2_multi(const StreamPlan &pl, const MultiRunViews &mv, const int4 *items,
-                         int n_items, cudaStream_t st, uint64_t *launches);
+int launch_stream2_multi(const StreamPlan &pl, const MultiRunViews &mv, const RunView *d_views,
+                         const int4 *items, int n_items, cudaStream_t st, uint64_t *launches);
 // once per updateEnergeticParticles call, before the stream2 launches
 int launch_stream2_coef(const RunView &r, cudaStream_t st, uint64_t *launches);
 int launch_stream2(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                    uint64_t *launches);
+// stream2m.cu -- the mirrored shape for any mu count from 4 to 64 (plan.mirror).  width: 0 automatic (by the slabs to stream at once), k >= 1 the k-th
+// number of list nodes per thread.  views, items: null, or as above for the
+// slabs of several runs, in device memory.
+// mirror_ok: the seed boundary is on and the mu grid uniform and symmetric.
+bool plan_stream2m(int N, int M, int m0, bool mirror_ok, int width, long long slabs,
+                   StreamPlan *plan);
+int stream2m_width_count(int M);
+int launch_stream2m(const RunView &r, const RunView *views, const int4 *items, int n_items,
+                    const StreamPlan &plan, cudaStream_t st, uint64_t *launches);
 // seedPopulationCheck alone in the FP32 form (rows renormalised)
 int launch_seed_check32(const RunView &r, cudaStream_t st, uint64_t *launches);
 

@@ -37,6 +37,7 @@ struct eprem_gpu_run {
   std::string skernel;  // eprem_gpu_stream_kernel's text
   eprem::NodePlan nplan{};
   int m0 = 0;
+  bool mirror_ok = false;  // seed boundary on, mu grid uniform and symmetric
   double norm_radius = 0, neg_beta = 0;
   double grid_dlnp = 0;  // dlnp of the momentum grid
   void *d_f = nullptr;
@@ -101,6 +102,7 @@ struct eprem_gpu_run {
   size_t cells() const {
     return (size_t)dims.num_streams * dims.num_nodes * dims.num_energies * dims.num_mu;
   }
+  long long slabs() const { return (long long)dims.num_streams * dims.num_energies; }
   size_t sn() const { return (size_t)dims.num_streams * dims.num_nodes; }
 };
 

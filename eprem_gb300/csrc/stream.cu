@@ -265,31 +265,40 @@ static int threads_for(int mmax) {
   }
 }
 
-// variant = kind + 8 * shape.  kind 0 automatic; FP32 form (stream2.cu):
+// variant = kind + 8 * shape.  kind 0 automatic; FP32 form:
 // 3 several list nodes per thread, 4 the same with packed fp32x2 arithmetic
 // (an odd mu half padded with a zero cell), 5 as 4 with the cell guards
-// resolved at compile time (M fills its bin, m0 = M/2), 6 and 7 as 5 with the
-// mu < 0 half in mirror order, one upwind coefficient per two cells (6 formed
-// on the sub-cycle loop, 7 from shared memory; both need the seed boundary)
-// -- the automatic kind is the first of 7, 5, 4, 3 that fits; shape 0 lets
-// plan_stream2 choose the CTA shape from N, k >= 1 names the k-th shape of
-// the mu bin.  The FP64 form has one kernel per stream length (stream64.cu, or
+// resolved at compile time (M fills its bin, m0 = M/2), 6 and 7 the mirrored
+// kernel of stream2m.cu (the mu < 0 half in mirror order, one upwind
+// coefficient per two cells; M = 20 or 40, and the seed boundary).  Shape 0
+// lets the planner choose from the sizes, k >= 1 names the k-th shape: of the
+// mu bin for 3 to 5, of the widths of M for 6 and 7.  The mirrored kernel
+// serves kinds 0, 4 and 5 with shape 0 too wherever it fits (mirror_ok: seed
+// boundary, and a uniform symmetric mu grid), and its widths follow the bin's
+// shapes there; the kernels of stream2.cu are left with the rest: runs without
+// the seed boundary, M < 4, other mu grids, shapes named by number.  96
+// streams x 50 E, ms of streaming in 30 sub-steps, stream2.cu's automatic
+// choice against it: M = 28, N = 1000 291 and 163; M = 33, N = 645, 26 E 179
+// and 59; M = 8, N = 1000 83 and 52; M = 64, N = 500 117 and 116.
+// The FP64 form has one kernel per stream length (stream64.cu, or
 // k_stream where a cluster of that one cannot hold the stream); variants 1 and
 // 2 name it there.
-int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, StreamPlan *plan) {
+int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool mirror_ok,
+                long long slabs, StreamPlan *plan) {
   if (precision == EPREM_FP32) {
     const int kind = variant % 8, shape = variant / 8;
     if (variant < 0 || kind == 1 || kind == 2) return EPREM_GPU_ERR_ARG;
-    if (kind == 6) return plan_stream2(N, M, m0, true, true, 1, bc, shape, plan);
-    if ((kind == 0 || kind == 7) && plan_stream2(N, M, m0, true, true, 2, bc, shape, plan) == 0)
+    const bool own = (M == 20 || M == 40) && 2 * m0 == M;
+    if (kind == 6 || kind == 7)
+      return own && plan_stream2m(N, M, m0, bc, shape, slabs, plan) ? 0 : EPREM_GPU_ERR_ARG;
+    const int old = stream2_shape_count(M);
+    if (kind != 3 && (shape == 0 || shape > old) &&
+        (kind != 5 || stream2_filled(M, m0)) &&
+        plan_stream2m(N, M, m0, mirror_ok, shape ? shape - old : 0, slabs, plan))
       return 0;
-    if (kind == 7) return EPREM_GPU_ERR_ARG;
-    if ((kind == 0 || kind == 5) && plan_stream2(N, M, m0, true, true, 0, bc, shape, plan) == 0)
-      return 0;
-    if ((kind == 0 || kind == 4) && plan_stream2(N, M, m0, true, false, 0, bc, shape, plan) == 0)
-      return 0;
-    if ((kind == 0 || kind == 3) && plan_stream2(N, M, m0, false, false, 0, bc, shape, plan) == 0)
-      return 0;
+    if ((kind == 0 || kind == 5) && plan_stream2(N, M, m0, true, true, shape, plan) == 0) return 0;
+    if ((kind == 0 || kind == 4) && plan_stream2(N, M, m0, true, false, shape, plan) == 0) return 0;
+    if ((kind == 0 || kind == 3) && plan_stream2(N, M, m0, false, false, shape, plan) == 0) return 0;
     return EPREM_GPU_ERR_ARG;
   }
   if (variant > 2) return EPREM_GPU_ERR_ARG;
