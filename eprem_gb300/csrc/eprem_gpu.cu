@@ -627,6 +627,15 @@ int eprem::ep_node_phase(eprem_gpu_run *r, const RunView &v) {
     });
     if (rc) return cuda_fail(cudaGetLastError(), "focusing/change launch");
   }
+  const bool shell = r->shell_on, drift = r->drift_on && r->drift_links;
+  if ((shell || drift) && perp_slice_fits(v, shell ? r->shell_L : 0, drift ? r->drift_L : 0)) {
+    rc = timed(r, EPREM_KERNEL_SHELL, [&] {
+      return launch_perp_slice(v, shell ? r->d_shell_ent : nullptr, r->shell_L, r->d_shell_del,
+                               drift ? r->d_drift_ent : nullptr, r->drift_L, r->d_drift_del,
+                               r->stream, &r->launches);
+    });
+    return rc ? cuda_fail(cudaGetLastError(), "shell diffusion / drift launch") : EPREM_GPU_OK;
+  }
   // (each perpendicular step swaps the run's two f buffers, which v, the
   // run's own view, sees)
   // DiffuseShellData after every stream's sub-step (src/energeticParticles.c:178-182)

@@ -126,6 +126,12 @@ int launch_shell_coef(const RunView &r, const int *news, double kperxkpar, void 
 // gather of DriftShellData (lists and fractions of launch_drift_coef)
 int launch_shell_diffuse(const RunView &r, const int *ent, int L, const void *del, void *out,
                          short *xout, cudaStream_t st, uint64_t *launches, bool drift = false);
+// Both operators of a sub-step in place, for slices (S rows of M cells) that
+// fit shared memory; ents null where an operator is off
+bool perp_slice_fits(const RunView &r, int shell_L, int drift_L);
+int launch_perp_slice(const RunView &r, const int *shell_ent, int shell_L, const void *shell_del,
+                      const int *drift_ent, int drift_L, const void *drift_del, cudaStream_t st,
+                      uint64_t *launches);
 // DriftShellData's fractions, Real[N][E][S][4], from r.curl and the positions
 int launch_drift_coef(const RunView &r, const int *news, void *del, cudaStream_t st,
                       uint64_t *launches);

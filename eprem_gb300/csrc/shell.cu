@@ -322,6 +322,272 @@ __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 4 : 2)
   }
 }
 
+// Both operators of a sub-step on one (node, energy) slice of all streams, in
+// shared memory: the hand-overs of a shell couple the streams' rows of one node
+// and energy alone, so a block that holds the slice's S rows of M cells applies
+// DiffuseShellData and then DriftShellData to them and writes them back in
+// place -- f crosses memory once each way for both, and no second f buffer is
+// needed.  Per operator a thread per row forms the row's new exponent and each
+// list entry's fraction taken to it (as k_shell_diffuse does per pair of
+// cells), then a thread per V cells of a row sums the entries in the
+// reference's order.  What bounds it is the gather's shared-memory loads and
+// the latency of the slice's rows (N E M cells apart); the lists' terms, formed
+// once per row, are half of its instructions at M = 20.  96 streams x 400 x 20 x
+// 20, FP32, a sub-step of both operators: 0.51 -> 0.14 ms.  For slices that fit
+// shared memory; k_shell_diffuse keeps the larger ones.
+// V cells of a row of f in place (a row starts at a multiple of V cells)
+template <int V, typename Real>
+__device__ __forceinline__ void ld_row(const Real *p, Real (&x)[V]) {
+  if constexpr (V == 4 && sizeof(Real) == 4) {
+    const float4 t = *reinterpret_cast<const float4 *>(p);
+    x[0] = t.x, x[1] = t.y, x[2] = t.z, x[3] = t.w;
+  } else if constexpr (V == 2 && sizeof(Real) == 4) {
+    const float2 t = *reinterpret_cast<const float2 *>(p);
+    x[0] = t.x, x[1] = t.y;
+  } else if constexpr (V == 2) {
+    const double2 t = *reinterpret_cast<const double2 *>(p);
+    x[0] = t.x, x[1] = t.y;
+  } else {
+#pragma unroll
+    for (int j = 0; j < V; j++) x[j] = p[j];
+  }
+}
+template <int V, typename Real>
+__device__ __forceinline__ void st_row(Real *p, const Real (&x)[V]) {
+  if constexpr (V == 4 && sizeof(Real) == 4)
+    *reinterpret_cast<float4 *>(p) = make_float4(x[0], x[1], x[2], x[3]);
+  else
+    st_vec<V>(p, x);
+}
+
+// four values of shared memory, 16-byte aligned
+__device__ __forceinline__ void ld_four(const float *p, float (&x)[4]) {
+  const float4 t = *reinterpret_cast<const float4 *>(p);
+  x[0] = t.x, x[1] = t.y, x[2] = t.z, x[3] = t.w;
+}
+__device__ __forceinline__ void ld_four(const double *p, double (&x)[4]) {
+  const double2 t = reinterpret_cast<const double2 *>(p)[0], u = reinterpret_cast<const double2 *>(p)[1];
+  x[0] = t.x, x[1] = t.y, x[2] = u.x, x[3] = u.y;
+}
+__device__ __forceinline__ void st_four(float *p, const float (&x)[4]) {
+  *reinterpret_cast<float4 *>(p) = make_float4(x[0], x[1], x[2], x[3]);
+}
+__device__ __forceinline__ void st_four(double *p, const double (&x)[4]) {
+  reinterpret_cast<double2 *>(p)[0] = make_double2(x[0], x[1]);
+  reinterpret_cast<double2 *>(p)[1] = make_double2(x[2], x[3]);
+}
+
+struct PerpOps {
+  const int *ent[2];    // lists: shell diffusion, drift; null where off
+  const void *del[2];   // fractions
+  int L[2];
+};
+
+// A row's term: its fraction (negative for a loss) at the row's exponent, and
+// where the source row starts.  A list shorter than L ends in zero fractions of
+// the row itself.
+template <typename Real>
+struct alignas(2 * sizeof(Real)) PerpTerm {
+  Real a;
+  int off;
+};
+
+template <typename Real>
+static size_t perp_smem(int S, int M, int L0, int L1) {
+  const int L = L0 > L1 ? L0 : L1;
+  // two buffers (rows at a pitch of whole 16 bytes), the slice's fractions of
+  // both operators, {fraction, list code} per entry, exponents
+  return 2 * sizeof(Real) * S * ((M + 3) / 4 * 4) + sizeof(PerpTerm<Real>) * S * L +
+         sizeof(Real) * 9 * S + sizeof(int) * S * (L0 + L1) + 2 * sizeof(int) * S;
+}
+
+constexpr int kPerpThreads = 256;
+
+// Places (row, column) of a table of `cols` columns, taken T apart from tid on:
+// stepped, not divided.
+struct Stepper {
+  int s, c, ds, dc, cols;
+  __device__ __forceinline__ Stepper(int tid, int T, int cols_) : cols(cols_) {
+    s = tid / cols;
+    c = tid - s * cols;
+    ds = T / cols;
+    dc = T - ds * cols;
+  }
+  __device__ __forceinline__ void next() {
+    s += ds;
+    c += dc;
+    if (c >= cols) c -= cols, ++s;
+  }
+};
+
+// A row's new exponent from its old one and the lowest that a gain asks for.
+__device__ __forceinline__ int new_exp(int x, int low) { return low < x ? clamp_exp(low) : x; }
+// ldexp_f of a fraction, by its exponent field where it stays a normal float.
+__device__ __forceinline__ float shifted(float a, int k) {
+  const int ex = (__float_as_int(a) >> 23) + k;
+  return a >= FLT_MIN && ex >= 1 && ex <= 254 ? __int_as_float(__float_as_int(a) + (k << 23))
+                                              : ldexp_f(a, k);
+}
+
+// V: cells of a row per access to memory (4, 2 or 1, as M divides).
+template <typename Real, int V>
+__global__ void __launch_bounds__(kPerpThreads, 6) k_perp_slice(RunView r, PerpOps ops) {
+  extern __shared__ __align__(16) unsigned char perp_sm[];
+  const int S = r.S, N = r.N, E = r.E, M = r.M, pitch = (M + 3) / 4 * 4;
+  const int Lmax = ops.L[0] > ops.L[1] ? ops.L[0] : ops.L[1];
+  Real *buf0 = reinterpret_cast<Real *>(perp_sm), *buf1 = buf0 + S * pitch;
+  PerpTerm<Real> *term = reinterpret_cast<PerpTerm<Real> *>(buf1 + S * pitch);  // [S][L]
+  Real *dl = reinterpret_cast<Real *>(term + S * Lmax);     // [S][5], [S][4] fractions
+  int *code = reinterpret_cast<int *>(dl + 9 * S);          // [S][L0], [S][L1]
+  int *xs = code + S * (ops.L[0] + ops.L[1]), *xw = xs + S;  // row exponents, new ones
+  const int tid = threadIdx.x, T = blockDim.x;
+  const size_t per_stream = (size_t)N * E * M;
+  const int nslices = (N - 1) * E;
+  const Stepper rows(tid, T, M / V), quads(tid, T, pitch / 4);
+  const Stepper lists[2] = {Stepper(tid, T, ops.L[0] > 0 ? ops.L[0] : 1),
+                            Stepper(tid, T, ops.L[1] > 0 ? ops.L[1] : 1)};
+#pragma unroll
+  for (int op = 0; op < 2; ++op)
+    for (int i = tid; i < S * ops.L[op]; i += T) code[op * S * ops.L[0] + i] = ops.ent[op][i];
+  for (int sl = blockIdx.x; sl < nslices; sl += gridDim.x) {
+    const int k = 1 + sl / E, e = sl - (sl / E) * E;  // node 0 hands nothing over
+    const size_t ke = (size_t)k * E + e;
+    Real *f = static_cast<Real *>(r.f) + ke * M;
+    __syncthreads();  // the last slice's rows have left
+#pragma unroll 2
+    for (Stepper i = rows; i.s < S; i.next()) {
+      Real x[V];
+      ld_row<V>(f + (size_t)i.s * per_stream + i.c * V, x);
+      if constexpr (V == 4) {
+        st_four(buf0 + i.s * pitch + i.c * V, x);
+      } else {
+#pragma unroll
+        for (int j = 0; j < V; j++) buf0[i.s * pitch + i.c * V + j] = x[j];
+      }
+    }
+    if constexpr (sizeof(Real) == 4)
+      for (int s = tid; s < S; s += T) xs[s] = xw[s] = r.fexp[((size_t)s * N + k) * E + e];
+    if (ops.ent[0])
+      for (int i = tid; i < 5 * S; i += T) dl[i] = static_cast<const Real *>(ops.del[0])[ke * S * 5 + i];
+    if (ops.ent[1])
+      for (int i = tid; i < 4 * S; i += T)
+        dl[5 * S + i] = static_cast<const Real *>(ops.del[1])[ke * S * 4 + i];
+    __syncthreads();
+#pragma unroll
+    for (int op = 0; op < 2; ++op) {
+      if (!ops.ent[op]) continue;
+      const bool drift = op == 1;
+      const int L = ops.L[op], ncoef = drift ? 4 : 5, mask = drift ? 3 : 7;
+      const Real *del = dl + op * 5 * S;
+      const int *cd0 = code + op * S * ops.L[0];
+      if constexpr (sizeof(Real) == 4) {  // xw[s]: xs[s], lowered by the row's gains
+        for (Stepper i = lists[op]; i.s < S; i.next()) {
+          const int cd = cd0[i.s * L + i.c];
+          if (cd < 0 || (cd & 7) >= 4) continue;
+          const float a = (float)del[(cd >> 3) * ncoef + (cd & mask)];
+          const int b = xs[cd >> 3] + 17 - ilogb_f(a);
+          if (a > 0.f && b < xs[i.s]) atomicMin(&xw[i.s], b);
+        }
+        __syncthreads();
+      }
+      for (Stepper i = lists[op]; i.s < S; i.next()) {
+        const int cd = cd0[i.s * L + i.c], from = cd < 0 ? i.s : cd >> 3;
+        Real a = Real(0);
+        if (cd >= 0) {
+          a = del[from * ncoef + (cd & mask)];
+          if constexpr (sizeof(Real) == 4)  // the source row taken to the new exponent
+            a = shifted(a, new_exp(xs[i.s], xw[i.s]) - xs[from]);
+          if ((cd & 7) >= 4) a = -a;
+        }
+        term[i.s * L + i.c] = PerpTerm<Real>{a, from * pitch};
+      }
+      __syncthreads();
+      for (Stepper i = quads; i.s < S; i.next()) {
+        const int c = i.c * 4;
+        Real acc[4] = {Real(0), Real(0), Real(0), Real(0)}, x[4];
+        const PerpTerm<Real> *t = term + i.s * L;
+#pragma unroll 4
+        for (int p = 0; p < L; ++p) {
+          const PerpTerm<Real> u = t[p];
+          ld_four(buf0 + u.off + c, x);
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[j] = sd_fma(u.a, x[j], acc[j]);
+        }
+        ld_four(buf0 + i.s * pitch + c, x);
+        if constexpr (sizeof(Real) == 4) {
+          const int d = new_exp(xs[i.s], xw[i.s]) - xs[i.s];
+          if (d)
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[j] = ldexp_f(x[j], d);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          x[j] = x[j] + acc[j];
+          if (nonfinite(x[j]) && c + j < M)
+            set_error(r, isnan(x[j]) ? EPREM_GPU_ERR_NAN : EPREM_GPU_ERR_INF, drift ? 7 : 6, i.s, k,
+                      e, c + j);
+        }
+        st_four(buf1 + i.s * pitch + c, x);
+      }
+      __syncthreads();
+      if constexpr (sizeof(Real) == 4) {
+        for (int s = tid; s < S; s += T) xs[s] = xw[s] = new_exp(xs[s], xw[s]);
+        __syncthreads();
+      }
+      Real *t = buf0;
+      buf0 = buf1;
+      buf1 = t;
+    }
+#pragma unroll 2
+    for (Stepper i = rows; i.s < S; i.next()) {
+      Real x[V];
+      if constexpr (V == 4) {
+        ld_four(buf0 + i.s * pitch + i.c * V, x);
+      } else {
+#pragma unroll
+        for (int j = 0; j < V; j++) x[j] = buf0[i.s * pitch + i.c * V + j];
+      }
+      st_row<V>(f + (size_t)i.s * per_stream + i.c * V, x);
+    }
+    if constexpr (sizeof(Real) == 4)
+      for (int s = tid; s < S; s += T) r.fexp[((size_t)s * N + k) * E + e] = (short)xs[s];
+  }
+}
+
+template <typename Real, int V>
+static cudaError_t launch_perp_as(const RunView &r, const PerpOps &ops, cudaStream_t st) {
+  const size_t smem = perp_smem<Real>(r.S, r.M, ops.L[0], ops.L[1]);
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_perp_slice<Real, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  // as many blocks as run at once: six by their registers, fewer by shared memory
+  const int fit = std::max(1, std::min(6, (int)(227 * 1024 / (smem + 1024))));
+  const int blocks = std::min((r.N - 1) * r.E, 152 * fit);
+  k_perp_slice<Real, V><<<blocks, kPerpThreads, smem, st>>>(r, ops);
+  return cudaGetLastError();
+}
+
+bool perp_slice_fits(const RunView &r, int shell_L, int drift_L) {
+  const size_t b = r.precision == EPREM_FP32 ? perp_smem<float>(r.S, r.M, shell_L, drift_L)
+                                             : perp_smem<double>(r.S, r.M, shell_L, drift_L);
+  return b <= 200 * 1024;
+}
+
+int launch_perp_slice(const RunView &r, const int *shell_ent, int shell_L, const void *shell_del,
+                      const int *drift_ent, int drift_L, const void *drift_del, cudaStream_t st,
+                      uint64_t *launches) {
+  const PerpOps ops{{shell_ent, drift_ent}, {shell_del, drift_del},
+                    {shell_ent ? shell_L : 0, drift_ent ? drift_L : 0}};
+  const cudaError_t e = r.precision == EPREM_FP32
+                            ? (r.M % 4 == 0   ? launch_perp_as<float, 4>(r, ops, st)
+                               : r.M % 2 == 0 ? launch_perp_as<float, 2>(r, ops, st)
+                                              : launch_perp_as<float, 1>(r, ops, st))
+                            : (r.M % 2 == 0 ? launch_perp_as<double, 2>(r, ops, st)
+                                            : launch_perp_as<double, 1>(r, ops, st));
+  ++*launches;
+  return e == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
+}
+
 int launch_shell_coef(const RunView &r, const int *news, double kperxkpar, void *del,
                       cudaStream_t st, uint64_t *launches) {
   const size_t SN = (size_t)r.S * r.N;
