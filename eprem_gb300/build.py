@@ -17,7 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libeprem_gpu.so")
-SOURCES = ["eprem_gpu.cu", "geometry.cu", "stream.cu", "stream64.cu", "node.cu", "node64.cu", "mhd.cu", "peak.cu", "node32.cu", "mas.cu", "stream2.cu", "stream2m.cu", "stream2m_1.cu", "stream2m_2.cu", "stream2m_3.cu", "stream2m_4.cu", "stream2m_5.cu", "stream2m_6.cu", "stream2m_7.cu", "mlp.cu", "surrogate.cu", "ensemble.cu", "surrogate_host.cu", "shell.cu"]
+SOURCES = ["eprem_gpu.cu", "geometry.cu", "stream.cu", "stream64.cu", "node.cu", "node64.cu", "mhd.cu", "peak.cu", "node32.cu", "node32_a.cu", "node32_b.cu", "mas.cu", "stream2.cu", "stream2m.cu", "stream2m_1.cu", "stream2m_2.cu", "stream2m_3.cu", "stream2m_4.cu", "stream2m_5.cu", "stream2m_6.cu", "stream2m_7.cu", "mlp.cu", "surrogate.cu", "ensemble.cu", "surrogate_host.cu", "shell.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
 # The background and node-motion kernels evaluate the reference's geometry

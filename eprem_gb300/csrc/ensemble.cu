@@ -9,6 +9,7 @@
 #include <string>
 #include <vector>
 
+#include "node32.cuh"
 #include "run.h"
 
 using namespace eprem;
@@ -179,6 +180,7 @@ struct eprem_gpu_ensemble {
   // lock-step: the slab lists of the merged streaming launches
   std::vector<int4 *> d_items;
   std::vector<RunView *> d_views;  // and their runs' views
+  std::vector<NodeBatch *> d_batches;  // the runs of the merged node launches
 };
 
 static void ensemble_drop_graph(eprem_gpu_ensemble *e) {
@@ -188,8 +190,10 @@ static void ensemble_drop_graph(eprem_gpu_ensemble *e) {
   e->graph = nullptr;
   for (int4 *p : e->d_items) cudaFree(p);
   for (RunView *p : e->d_views) cudaFree(p);
+  for (NodeBatch *p : e->d_batches) cudaFree(p);
   e->d_items.clear();
   e->d_views.clear();
+  e->d_batches.clear();
 }
 
 extern "C" int eprem_gpu_ensemble_destroy(eprem_gpu_ensemble *e) {
@@ -295,9 +299,8 @@ extern "C" int eprem_gpu_ensemble_autotune(eprem_gpu_ensemble *e, int *chosen_va
 // share a packed streaming kernel (mu bin, CTA shape, cluster size, guards),
 // the group's (run, stream, energy) slabs ordered by their estimated work,
 // longest first, so the slabs of small runs fill the tails of large ones --
-// and the node phases -- one focusing and one change launch per group of
-// runs of one mu count over all their row and node blocks, the other runs'
-// own launches; all on the ensemble's stream.  Each slab and
+// and the node phases -- one launch per group of runs of one mu count over all
+// their nodes, the other runs' own launches; all on the ensemble's stream.  Each slab and
 // row is computed by the same code as in a run's own update: the results are
 // the runs' own, bit for bit.  Needs the same numEpSteps in every run.
 namespace {
@@ -398,44 +401,58 @@ static int ensemble_capture_lockstep(eprem_gpu_ensemble *e) {
     CK(cudaMemcpy(dv, views[gi].v, sizeof(RunView) * groups[gi].runs.size(),
                   cudaMemcpyHostToDevice));
   }
-  // node phases: runs of one mu count in the plain form, focusing and change
-  // both on, in two launches per sub-step over all their (run, block) items
+  // node phases: runs of one mu count in the plain form, one launch per sub-step
+  // over all their nodes (focusing and change on or off alike in all of them)
   struct NodeGroup {
-    int M;
+    int M, focus, change;
     std::vector<int> runs;
-    NodeRunViews views;
+    NodePlan plan;
+    int blocks = 0;
+    NodeBatch *d = nullptr;
   };
   std::vector<NodeGroup> ngroups;
   std::vector<char> node_grouped(n, 0);
   for (int i = 0; i < n; i++) {
     eprem_gpu_run *r = e->runs[i];
-    if (r->node_mode != EPREM_NODE_PHASE_REFERENCE || !r->nplan.fast32 || !r->v.use_focus ||
-        !r->v.use_change || r->shell_on || r->drift_on)
+    if (r->node_mode != EPREM_NODE_PHASE_REFERENCE || !r->nplan.fast32 ||
+        !(r->v.use_focus || r->v.use_change) || r->shell_on || r->drift_on)
       continue;
     NodeGroup *grp = nullptr;
     for (auto &ng : ngroups)
-      if (ng.M == r->dims.num_mu && (int)ng.runs.size() < kMultiRuns) grp = &ng;
+      if (ng.M == r->dims.num_mu && ng.focus == r->v.use_focus && ng.change == r->v.use_change &&
+          (int)ng.runs.size() < kMultiRuns)
+        grp = &ng;
     if (!grp) {
       ngroups.push_back(NodeGroup{});
       grp = &ngroups.back();
       grp->M = r->dims.num_mu;
+      grp->focus = r->v.use_focus;
+      grp->change = r->v.use_change;
     }
     grp->runs.push_back(i);
   }
   for (auto &ng : ngroups) {
-    ng.views.n = 0;
     if (ng.runs.size() < 2) continue;  // a lone run keeps its own launches
-    ng.views.n = (int)ng.runs.size();
-    ng.views.foff[0] = ng.views.coff[0] = 0;
-    for (int j = 0; j < ng.views.n; j++) {
-      eprem_gpu_run *r = e->runs[ng.runs[j]];
-      ng.views.v[j] = r->v;
-      int nf = 0, nc = 0;
-      node32_blocks(r->v, &nf, &nc);
-      ng.views.foff[j + 1] = ng.views.foff[j] + nf;
-      ng.views.coff[j + 1] = ng.views.coff[j] + nc;
-      node_grouped[ng.runs[j]] = 1;
+    size_t nodes = 0;
+    for (int i : ng.runs) nodes += e->runs[i]->sn();
+    std::vector<const RunView *> vs;
+    std::vector<NodePlan> pls;
+    for (int i : ng.runs) {
+      eprem_gpu_run *r = e->runs[i];
+      NodePlan pl = r->nplan;  // the shape for all the group's nodes
+      if (plan_node32(r->dims.num_energies, r->dims.num_mu, nodes, &pl))
+        return fail(EPREM_GPU_ERR_ARG, "ensemble node plan");
+      vs.push_back(&r->v);
+      pls.push_back(pl);
+      node_grouped[i] = 1;
     }
+    std::vector<NodeBatch> nb(1);
+    if (node32_batch(vs, pls, nb.data(), &ng.plan))
+      return fail(EPREM_GPU_ERR_ARG, "ensemble node batch");
+    ng.blocks = nb[0].off[nb[0].n];
+    CK(cudaMalloc(&ng.d, sizeof(NodeBatch)));
+    e->d_batches.push_back(ng.d);
+    CK(cudaMemcpy(ng.d, nb.data(), sizeof(NodeBatch), cudaMemcpyHostToDevice));
   }
   std::vector<bool> saved(n);
   std::vector<cudaStream_t> own(n);
@@ -469,8 +486,8 @@ static int ensemble_capture_lockstep(eprem_gpu_ensemble *e) {
     for (int i : solo)
       if (!rc && err == cudaSuccess) rc = ep_stream_phase(e->runs[i], e->runs[i]->v);
     for (auto &ng : ngroups)
-      if (ng.views.n && !rc && err == cudaSuccess &&
-          launch_node32_multi(e->runs[ng.runs[0]]->nplan, ng.views, e->origin,
+      if (ng.d && !rc && err == cudaSuccess &&
+          launch_node32_multi(ng.plan, e->runs[ng.runs[0]]->v, ng.blocks, ng.d, e->origin,
                               &e->runs[ng.runs[0]]->launches))
         err = cudaGetLastError();
     for (int i = 0; i < n && !rc && err == cudaSuccess; i++)

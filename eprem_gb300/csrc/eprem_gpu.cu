@@ -160,7 +160,7 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
   const bool fast64 = dims->precision == EPREM_FP64 && params->adiabatic_focus_alg <= 2 &&
                       params->adiabatic_change_alg <= 2;
   if (!prc)
-    prc = fast32   ? plan_node32(E, M, &r->nplan)
+    prc = fast32   ? plan_node32(E, M, (size_t)S * N, &r->nplan)
           : fast64 ? plan_node64(E, M, params->adiabatic_focus_alg, &r->nplan)
                    : plan_node(dims->precision, E, M, &r->nplan);
   r->nplan.fast32 = fast32 ? 1 : 0;

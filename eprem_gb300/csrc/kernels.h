@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <vector>
 
 #include "common.cuh"
 
@@ -85,23 +86,18 @@ int launch_node(const RunView &r, const NodePlan &plan, cudaStream_t st, uint64_
 // node64.cu -- FP64-form focusing + change (Euler and RK3 operators)
 int plan_node64(int E, int M, int focus_alg, NodePlan *plan);
 int launch_node64(const RunView &r, const NodePlan &plan, cudaStream_t st, uint64_t *launches);
-// node32.cu -- FP32-form focusing + change (Euler operators)
-int plan_node32(int E, int M, NodePlan *plan);
+// node32.cu -- FP32-form focusing + change (Euler operators); nodes: the run's
+int plan_node32(int E, int M, size_t nodes, NodePlan *plan);
 int launch_node32(const RunView &r, const NodePlan &plan, cudaStream_t st, uint64_t *launches);
 // once per updateEnergeticParticles call, before the first launch_node32
 int launch_node32_setup(const RunView &r, cudaStream_t st, uint64_t *launches);
-// The node phase (focusing then change, both on) of several runs of one mu
-// count and one plan in two launches; a run's own launches are the same
-// kernels over one view.  foff / coff: each run's first focusing / change
-// CTA (prefix sums of node32_blocks), n runs.
-struct NodeRunViews {
-  RunView v[kMultiRuns];
-  int foff[kMultiRuns + 1], coff[kMultiRuns + 1];
-  int n;
-};
-void node32_blocks(const RunView &r, int *focus_blocks, int *change_blocks);
-int launch_node32_multi(const NodePlan &pl, const NodeRunViews &nv, cudaStream_t st,
-                        uint64_t *launches);
+// The node phase of several runs of one mu count in one launch: node32_batch
+// fills the batch (then copied to the device) and the launch's plan.
+struct NodeBatch;
+int node32_batch(const std::vector<const RunView *> &views, const std::vector<NodePlan> &plans,
+                 NodeBatch *nb, NodePlan *pl);
+int launch_node32_multi(const NodePlan &pl, const RunView &first, int blocks,
+                        const NodeBatch *batch, cudaStream_t st, uint64_t *launches);
 
 // mhd.cu -- updateMhd (analytic), moveNodes, omnidirectional flux, f conversion
 struct MhdParams {
