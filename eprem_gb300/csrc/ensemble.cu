@@ -11,6 +11,7 @@
 
 #include "node32.cuh"
 #include "run.h"
+#include "stream2m.cuh"
 
 using namespace eprem;
 
@@ -179,7 +180,7 @@ struct eprem_gpu_ensemble {
   int chains = -1;  // < 0 lock-step with merged streaming; 0 one branch per run; k serial chains
   // lock-step: the slab lists of the merged streaming launches
   std::vector<int4 *> d_items;
-  std::vector<RunView *> d_views;  // and their runs' views
+  std::vector<Stream2mView *> d_views;  // and their runs' views
   std::vector<NodeBatch *> d_batches;  // the runs of the merged node launches
 };
 
@@ -189,7 +190,7 @@ static void ensemble_drop_graph(eprem_gpu_ensemble *e) {
   e->exec = nullptr;
   e->graph = nullptr;
   for (int4 *p : e->d_items) cudaFree(p);
-  for (RunView *p : e->d_views) cudaFree(p);
+  for (Stream2mView *p : e->d_views) cudaFree(p);
   for (NodeBatch *p : e->d_batches) cudaFree(p);
   e->d_items.clear();
   e->d_views.clear();
@@ -395,11 +396,12 @@ static int ensemble_capture_lockstep(eprem_gpu_ensemble *e) {
     e->d_items.push_back(d);
     CK(cudaMemcpy(d, flat.data(), flat.size() * sizeof(int4), cudaMemcpyHostToDevice));
     n_items[gi] = (int)flat.size();
-    RunView *dv = nullptr;
-    CK(cudaMalloc(&dv, sizeof(RunView) * groups[gi].runs.size()));
+    std::vector<Stream2mView> sv;
+    for (size_t j = 0; j < groups[gi].runs.size(); j++) sv.push_back(stream2m_view(views[gi].v[j]));
+    Stream2mView *dv = nullptr;
+    CK(cudaMalloc(&dv, sizeof(Stream2mView) * sv.size()));
     e->d_views.push_back(dv);
-    CK(cudaMemcpy(dv, views[gi].v, sizeof(RunView) * groups[gi].runs.size(),
-                  cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dv, sv.data(), sizeof(Stream2mView) * sv.size(), cudaMemcpyHostToDevice));
   }
   // node phases: runs of one mu count in the plain form, one launch per sub-step
   // over all their nodes (focusing and change on or off alike in all of them)

@@ -53,7 +53,9 @@ struct MultiRunViews {
   RunView v[kMultiRuns];
   int m0[kMultiRuns];
 };
-int launch_stream2_multi(const StreamPlan &pl, const MultiRunViews &mv, const RunView *d_views,
+struct Stream2mView;
+int launch_stream2_multi(const StreamPlan &pl, const MultiRunViews &mv,
+                         const Stream2mView *d_views,
                          const int4 *items, int n_items, cudaStream_t st, uint64_t *launches);
 // once per updateEnergeticParticles call, before the stream2 launches
 int launch_stream2_coef(const RunView &r, cudaStream_t st, uint64_t *launches);
@@ -66,7 +68,9 @@ int launch_stream2(const RunView &r, const StreamPlan &plan, int m0, cudaStream_
 bool plan_stream2m(int N, int M, int m0, bool mirror_ok, int width, long long slabs,
                    StreamPlan *plan);
 int stream2m_width_count(int M);
-int launch_stream2m(const RunView &r, const RunView *views, const int4 *items, int n_items,
+struct Stream2mView;
+Stream2mView stream2m_view(const RunView &r);
+int launch_stream2m(const RunView &r, const Stream2mView *views, const int4 *items, int n_items,
                     const StreamPlan &plan, cudaStream_t st, uint64_t *launches);
 // seedPopulationCheck alone in the FP32 form (rows renormalised)
 int launch_seed_check32(const RunView &r, cudaStream_t st, uint64_t *launches);

@@ -899,7 +899,8 @@ static cudaError_t launch_stream2_multi_t(const StreamPlan &pl, const MultiRunVi
                         st, args);
 }
 
-int launch_stream2_multi(const StreamPlan &pl, const MultiRunViews &mv, const RunView *d_views,
+int launch_stream2_multi(const StreamPlan &pl, const MultiRunViews &mv,
+                         const Stream2mView *d_views,
                          const int4 *items, int n_items, cudaStream_t st, uint64_t *launches) {
   if (!pl.packed || n_items <= 0) return EPREM_GPU_ERR_ARG;
   if (pl.mirror) return launch_stream2m(mv.v[0], d_views, items, n_items, pl, st, launches);

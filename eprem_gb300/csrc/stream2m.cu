@@ -2,7 +2,7 @@
 // instances are compiled in stream2m_1.cu to stream2m_7.cu.
 #include <cmath>
 
-#include "kernels.h"
+#include "stream2m.cuh"
 #include "stream2m_list.h"
 
 namespace eprem {
@@ -112,7 +112,13 @@ bool plan_stream2m(int N, int M, int m0, bool mirror_ok, int width, long long sl
   return true;
 }
 
-int launch_stream2m(const RunView &r, const RunView *views, const int4 *items, int n_items,
+Stream2mView stream2m_view(const RunView &r) {
+  return Stream2mView{r.N,    r.E,         r.M,      r.check_seed, (float *)r.f, r.fexp, r.mugrid,
+                      r.ec,   r.list,      r.list_size, r.ds_min,  r.scoef,      r.status, r.dt,
+                      r.dmu,  r.max_subcycles, r.s_base};
+}
+
+int launch_stream2m(const RunView &r, const Stream2mView *views, const int4 *items, int n_items,
                     const StreamPlan &pl, cudaStream_t st, uint64_t *launches) {
   const int P = pairs_of(pl.mmax);
   const bool extra = extra_of(pl.mmax);
@@ -138,7 +144,7 @@ int launch_stream2m(const RunView &r, const RunView *views, const int4 *items, i
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  RunView rv = r;
+  Stream2mView rv = stream2m_view(r);
   void *args[] = {&rv, &views, &items};
   *launches += 1;
   return cudaLaunchKernelExC(&cfg, kern, args) == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;

@@ -36,6 +36,26 @@ namespace cg = cooperative_groups;
 
 namespace eprem {
 
+// What the kernel reads of a run (a layout of its own: the kernel sits at 255
+// registers, and unrelated fields of RunView moving about cost it 5 %).
+struct Stream2mView {
+  int N, E, M, check_seed;
+  float *f;
+  short *fexp;
+  const double *mugrid;
+  const EnergyConsts *ec;
+  const int *list, *list_size;
+  const double *ds_min;
+  const float4 *scoef;
+  DevStatus *status;
+  double dt, dmu;
+  int max_subcycles, s_base;
+};
+__device__ __forceinline__ void set_error(const Stream2mView &r, int code, int s, int k, int e,
+                                          int m) {
+  set_error(r.status, code, 1, s + r.s_base, k, e, m);
+}
+
 // Shared memory per thread, in floats: rows at a pitch of an odd number of
 // 16-byte units (8 lanes' float4 accesses fall into distinct banks), the
 // coefficients at an odd number of 8-byte units.
@@ -83,7 +103,8 @@ __device__ __forceinline__ void s2m_put_far(float *dst, const float2 (&h)[P], fl
 // cluster i of the launch takes slab items[i] = (run, stream, energy).
 template <int P, bool EXTRA, int NPT>
 __global__ void __launch_bounds__(256, 1)
-    k_stream2m(const __grid_constant__ RunView r0, const RunView *views, const int4 *items) {
+    k_stream2m(const __grid_constant__ Stream2mView r0, const Stream2mView *views,
+               const int4 *items) {
   using Lay = S2mLayout<P, EXTRA, NPT>;
   constexpr int PITCH = Lay::kPitch;
   extern __shared__ __align__(16) float sm2m[];
@@ -93,14 +114,14 @@ __global__ void __launch_bounds__(256, 1)
   const int T = blockDim.x, W = T >> 5;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int s = blockIdx.y, e = r0.E - 1 - (int)blockIdx.z;
-  const RunView *rp = &r0;
+  const Stream2mView *rp = &r0;
   if (items) {
     const int4 it = items[blockIdx.x / C];
     rp = views + it.x;
     s = it.y;
     e = it.z;
   }
-  const RunView &r = *rp;
+  const Stream2mView &r = *rp;
   const int N = r.N, M = r.M, E = r.E;
   const int nh = M / 2;                          // cells per half
   const bool odd_half = EXTRA && nh == 2 * P + 1;  // the half's last slot is l, r
@@ -112,7 +133,7 @@ __global__ void __launch_bounds__(256, 1)
   const double dtMin = 0.4 * r.ds_min[s] * ec.vgrid_i;
   const double nst = floor(r.dt / dtMin + 1.0);
   if (!(nst <= (double)r.max_subcycles)) {
-    if (crank == 0 && tid == 0) set_error(r, EPREM_GPU_ERR_SUBCYCLES, 1, s, -1, e, -1);
+    if (crank == 0 && tid == 0) set_error(r, EPREM_GPU_ERR_SUBCYCLES, s, -1, e, -1);
     return;
   }
   const int nsteps = (int)nst;
@@ -164,7 +185,7 @@ __global__ void __launch_bounds__(256, 1)
       const int k = r.list[sN + il];
       const float4 c = sc[il];
       // slot j: cells nh - 1 - j and M - nh + j
-      const float *row = reinterpret_cast<const float *>(r.f) + ((sN + k) * E + e) * M;
+      const float *row = r.f + ((sN + k) * E + e) * M;
       const float *up = row + (M - nh), *dn = row + nh - 1;
       float mx = 0.f;
       if constexpr (!EXTRA && P % 2 == 0) {  // M = 4 P: rows in 16-byte pieces
@@ -312,7 +333,7 @@ __global__ void __launch_bounds__(256, 1)
       __syncwarp();
       if (W > 1 && !timed_out && !halo_wait(&s_bar[ph][warp], (uint32_t)(step >> 1) & 1u)) {
         timed_out = true;  // reported once; later waits are skipped
-        if (lane == 0) set_error(r, EPREM_GPU_ERR_CUDA, 1, s, -1, e, -1);
+        if (lane == 0) set_error(r, EPREM_GPU_ERR_CUDA, s, -1, e, -1);
       }
     }
     const float4 *srcL = reinterpret_cast<const float4 *>(rowL(ph, tid + 2));
@@ -402,7 +423,7 @@ __global__ void __launch_bounds__(256, 1)
       const int k = r.list[sN + il];
       int code = 0;
       auto out = [&](float v, int m) {
-        if (bad_value(v, &code)) set_error(r, code, 1, s, k, e, m);
+        if (bad_value(v, &code)) set_error(r, code, s, k, e, m);
         return v < FLT_MIN ? FLT_MIN : v;
       };
 #pragma unroll
@@ -418,7 +439,7 @@ __global__ void __launch_bounds__(256, 1)
       const int kfirst = (il == 0) ? 0 : r.list[sN + il - 1] + 1;
       for (int kk = kfirst; kk <= k; ++kk) {
         r.fexp[(sN + kk) * E + e] = (short)K;
-        float *row = reinterpret_cast<float *>(r.f) + ((sN + kk) * E + e) * M;
+        float *row = r.f + ((sN + kk) * E + e) * M;
         float *up = row + (M - nh), *dn = row + nh - 1;
         if constexpr (!EXTRA && P % 2 == 0) {
           float4 *op = reinterpret_cast<float4 *>(row);
