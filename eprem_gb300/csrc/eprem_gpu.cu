@@ -17,6 +17,7 @@
 #include <string>
 #include <vector>
 
+#include "math64.cuh"
 #include "run.h"
 
 using namespace eprem;
@@ -191,6 +192,7 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
   if (e == cudaSuccess) e = dalloc(&r->d_mugrid32, (size_t)M);
   if (e == cudaSuccess && fast32) e = dalloc(&r->d_coef32, SN);
   if (e == cudaSuccess && fast64) e = dalloc(&r->d_coef64, SN);
+  if (e == cudaSuccess && fast64) e = dalloc(&r->d_math64, kMath64Size);
   // FP32 streaming coefficients (any FP32 run may be tuned to stream2.cu)
   if (e == cudaSuccess && dims->precision == EPREM_FP32 && params->use_parallel_diffusion > 0)
     e = dalloc(&r->d_scoef, SN * (size_t)dims->num_energies);
@@ -241,6 +243,10 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
     e = cudaMemcpyAsync(r->d_mugrid, grids->mugrid, M * sizeof(double), cudaMemcpyHostToDevice, r->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(r->d_mugrid32, mu32.data(), M * sizeof(float), cudaMemcpyHostToDevice, r->stream);
+  static const std::vector<double> math64 = math64_tables();
+  if (e == cudaSuccess && r->d_math64)
+    e = cudaMemcpyAsync(r->d_math64, math64.data(), kMath64Size * sizeof(double),
+                        cudaMemcpyHostToDevice, r->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(r->stream);
   if (e != cudaSuccess) {
     eprem_gpu_destroy(r);
@@ -264,6 +270,7 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
   v.mugrid32 = r->d_mugrid32;
   v.coef32 = r->d_coef32;
   v.coef64 = r->d_coef64;
+  v.math64 = r->d_math64;
   v.scoef = r->d_scoef;
   v.ec = r->d_ec;
   v.list = r->d_list;
@@ -325,6 +332,7 @@ extern "C" int eprem_gpu_destroy(eprem_gpu_run *r) {
   cudaFree(r->d_reject);
   cudaFree(r->d_coef32);
   cudaFree(r->d_coef64);
+  cudaFree(r->d_math64);
   cudaFree(r->d_scoef);
   cudaFree(r->d_ec);
   cudaFree(r->d_list);

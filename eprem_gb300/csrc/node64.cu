@@ -13,15 +13,17 @@
 //   * a cell takes two multiply-adds, f - q f_up + q' f_up' , the upwind cell
 //     chosen by the sign bit of q (no FP64 compare), floors and NaN checks by
 //     the bits of the high word;
-//   * ln and exp run over the CTA's cells in order, every lane busy.
+//   * ln and exp (math64.cuh) run over the CTA's cells in order, every lane busy.
 // A CTA holds G whole nodes in shared memory; focusing takes a (node, energy)
 // row per thread, change a (node, mu) column, rows at an odd pitch (no bank
 // conflicts either way).
-// Per launch on a GB300 (node.cu before): 6 x 1000 x 50 x 40, 3.71 -> 1.45 ms (76
-// FP64 operations a cell, of which ln and exp are 57); 24 x 400 x 20 x 20, 1.33
-// -> 0.40 ms; third order, 24 x 200 x 20 x 20, 1.80 -> 0.60 ms.
+// Per launch on a GB300 (node.cu before; with CUDA's log and exp between): 6 x
+// 1000 x 50 x 40, 3.71 -> 1.45 -> 0.93 ms (48 FP64 slots a cell); 24 x 400 x 20 x
+// 20, 1.33 -> 0.40 -> 0.24 ms; third order, 24 x 200 x 20 x 20, 1.80 -> 0.60 ->
+// 0.52 ms.
 #include "common.cuh"
 #include "kernels.h"
+#include "math64.cuh"
 
 namespace eprem {
 
@@ -174,7 +176,7 @@ __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) 
       v = floored(v);
     }
     if (change)
-      f[row * pitch + m] = log(v);
+      f[row * pitch + m] = ln64(v, r.math64);
     else
       fg[i] = v;
   }
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) 
   for (int i = tid; i < Gv * EM; i += T) {
     const int row = i / M, m = i - row * M, n = row / E;
     if (!nc[n].ok) continue;
-    const double v = exp(f[row * pitch + m]);
+    const double v = exp64(f[row * pitch + m], r.math64);
     if (not_finite(v)) {
       const size_t g = g0 + n;
       set_error(r, nan_or_inf(v), 3, (int)(g / N), (int)(g % N), row - n * E, m);

@@ -46,6 +46,7 @@ struct eprem_gpu_run {
   float *d_mugrid32 = nullptr;
   eprem::NodeCoef32 *d_coef32 = nullptr;
   eprem::NodeCoef64 *d_coef64 = nullptr;
+  double *d_math64 = nullptr;
   float4 *d_scoef = nullptr;
   eprem::EnergyConsts *d_ec = nullptr;
   int *d_list = nullptr, *d_list_size = nullptr;

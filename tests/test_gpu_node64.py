@@ -60,3 +60,28 @@ def test_rates_outside_and_inside_the_float_prefilter(scale, oracle_lib):
         if scale < 1.0:
             nodes[abi.NODE["BMAG"], 5:40] = 1.0  # no focusing by dlnB/ds either
     _check(W.custom(1, 1, 60, 8, 10, num_ep_steps=2), oracle_lib, tweak)
+
+
+def test_logarithm_and_exponential(oracle_lib):
+    """Nodes whose rates are zero take no sub-cycle, so the change writes back
+    exp(ln f): ln to half a unit in its last place (7e-17 below 1) and exp to 0.7
+    of one, with room for a tenth of each, over the whole range of f."""
+    w = W.custom(1, 1, 40, 8, 12, num_ep_steps=1, use_parallel_diffusion=0,
+                 use_adiabatic_focus=0, check_seed_population=0)
+    d, g, f, nodes = primed_state(w, oracle_lib)
+    for fld in ("DLNB", "DLNN", "DUPAR"):
+        nodes[abi.NODE[fld]] = 0.0
+    rng = np.random.default_rng(3)
+    f = np.exp(rng.uniform(-700.0, 700.0, f.size))
+    f[::7] = np.exp(rng.uniform(-2.0, 2.0, f[::7].size))
+    f[0::1001] = np.finfo(np.float64).tiny
+    run = EpremRun(d, w.params, g)
+    run.upload_f(f)
+    run.upload_nodes(nodes)
+    run.update_energetic_particles(0.0)
+    assert run.read_stats().max_subcycles_change == 0
+    out = run.download_f()
+    run.close()
+    eps = 2.0 ** -53
+    bound = 1.1 * (np.maximum(np.spacing(np.abs(np.log(f))) / 2.0, 7e-17) + 1.4 * eps) + eps
+    assert np.all(np.abs(out - f) <= bound * f)
