@@ -49,6 +49,7 @@ struct EnergyConsts {
   float dvi32;           // vgrid_i[e+1] - vgrid_i[e-1] (0 at the ends), from FP64
   int seed_k;            // FP32 streaming seeds are held as seed * 2^seed_k, so that
                          // the energy-only factor of sepSeedFunction is near 1
+  double seed_c;         // that factor times 2^seed_k, in [1, 2) unless it underflows
   double two_vi;         // 2 / vgrid (the focusing speed's factor of DuPar)
   double drift_factor;   // (1/om1) p v / 3 of driftVelocity (src/energeticParticles.c:
                          // 210-246), p = exp(lnpmin + E dlnp); 0 without drift

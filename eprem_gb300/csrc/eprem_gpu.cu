@@ -233,6 +233,7 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
     // the energy-only factor of sepSeedFunction, normalised to [1, 2) by 2^seed_k
     const double ce = norm_j0 * ec[i].seed_power * ec[i].seed_exp / p.bf_xi / (2.0 * ec[i].egrid);
     ec[i].seed_k = (std::isfinite(ce) && ce >= DBL_MIN) ? -ilogb(ce) : 1022;
+    ec[i].seed_c = ldexp(ce, ec[i].seed_k);
   }
   std::vector<float> mu32(M);
   for (int m = 0; m < M; m++) mu32[m] = (float)grids->mugrid[m];

@@ -220,13 +220,12 @@ int launch_geometry(const RunView &r, cudaStream_t st, double norm_radius, doubl
                     int mfp_type, double mfp_power, double bs_au, uint64_t *launches,
                     bool node_rates) {
   const size_t SN = (size_t)r.S * r.N;
-  // 64 threads a CTA: FP64 latency bounds a node's chain, and a small run has
-  // no more than a warp or two per SM
-  const int blocks = (int)std::min<size_t>((SN + 63) / 64, 152 * 64);
+  const int t = node_threads(SN);
+  const int blocks = (int)std::min<size_t>((SN + t - 1) / t, 152 * 64);
   if (node_rates && r.coef64)
-    k_node_prep<true><<<blocks, 64, 0, st>>>(r, norm_radius, neg_beta, mfp_type, mfp_power, bs_au);
+    k_node_prep<true><<<blocks, t, 0, st>>>(r, norm_radius, neg_beta, mfp_type, mfp_power, bs_au);
   else
-    k_node_prep<false><<<blocks, 64, 0, st>>>(r, norm_radius, neg_beta, mfp_type, mfp_power, bs_au);
+    k_node_prep<false><<<blocks, t, 0, st>>>(r, norm_radius, neg_beta, mfp_type, mfp_power, bs_au);
   size_t smem = (size_t)r.N * (3 * sizeof(double) + sizeof(int));
   // per launch: runs of different sizes share the kernel's attribute
   if (cudaFuncSetAttribute(k_stream_list, cudaFuncAttributeMaxDynamicSharedMemorySize,

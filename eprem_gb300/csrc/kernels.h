@@ -8,6 +8,11 @@
 
 namespace eprem {
 
+// Threads per CTA of a kernel with an FP64 chain per node (one thread each): an
+// SM's warps share two FP64 lanes, so few nodes want a warp to an SM, not eight
+// (k_update_mhd, 1440 nodes: 50 us in CTAs of 256 threads, 28 of 32).
+inline int node_threads(size_t nodes) { return nodes <= (size_t)152 * 32 * 8 ? 32 : 128; }
+
 // geometry.cu
 // node_rates: also the node coefficients and sub-cycle counts (added to the
 // statistics) of the FP64 form's node64.cu, once per updateEnergeticParticles

@@ -252,21 +252,25 @@ __global__ void k_mas_move_nodes(RunView r, MasView mv, double dt) {
   }
 }
 
-static int mas_grid(size_t n) {
-  size_t b = (n + 127) / 128;
+static int mas_grid(size_t n, int threads) {
+  const size_t b = (n + threads - 1) / threads;
   return (int)(b > 152 * 64 ? 152 * 64 : (b ? b : 1));
 }
 
 int launch_mas_update_mhd(const RunView &r, const MasView &mv, double t_del, cudaStream_t st,
                           uint64_t *launches) {
-  k_mas_update_mhd<<<mas_grid((size_t)r.S * r.N), 128, 0, st>>>(r, mv, t_del);
+  const size_t n = (size_t)r.S * r.N;
+  const int t = node_threads(n);
+  k_mas_update_mhd<<<mas_grid(n, t), t, 0, st>>>(r, mv, t_del);
   *launches += 1;
   return cudaGetLastError() == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }
 
 int launch_mas_move_nodes(const RunView &r, const MasView &mv, double dt, cudaStream_t st,
                           uint64_t *launches) {
-  k_mas_move_nodes<<<mas_grid((size_t)r.S * r.N), 128, 0, st>>>(r, mv, dt);
+  const size_t n = (size_t)r.S * r.N;
+  const int t = node_threads(n);
+  k_mas_move_nodes<<<mas_grid(n, t), t, 0, st>>>(r, mv, dt);
   *launches += 1;
   return cudaGetLastError() == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }

@@ -9,6 +9,8 @@
 //                  branch of delrFlow (src/flow.c:162-196)
 //   k_omni_flux  : computeFlux without its unit scale (src/unifiedOutput.c:153-180)
 // All FP64, one thread per node.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -235,9 +237,15 @@ static int grid_for(size_t n) {
   return (int)(b > 152 * 32 ? 152 * 32 : (b ? b : 1));
 }
 
+static int node_grid(size_t n, int threads) {
+  return (int)std::min<size_t>((n + threads - 1) / threads, 152 * 64);
+}
+
 int launch_update_mhd(const RunView &r, const MhdParams &p, double tg, cudaStream_t st,
                       uint64_t *launches, const double *tg_dev) {
-  k_update_mhd<<<grid_for((size_t)r.S * r.N), 256, 0, st>>>(r, p, tg, tg_dev);
+  const size_t n = (size_t)r.S * r.N;
+  const int t = node_threads(n);
+  k_update_mhd<<<node_grid(n, t), t, 0, st>>>(r, p, tg, tg_dev);
   *launches += 1;
   return cudaGetLastError() == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }
@@ -253,7 +261,9 @@ int launch_advance_time(double *t_dev, double dt, cudaStream_t st, uint64_t *lau
 }
 
 int launch_move_nodes(const RunView &r, double dt, cudaStream_t st, uint64_t *launches) {
-  k_move_nodes<<<grid_for((size_t)r.S * r.N), 256, 0, st>>>(r, dt);
+  const size_t n = (size_t)r.S * r.N;
+  const int t = node_threads(n);
+  k_move_nodes<<<node_grid(n, t), t, 0, st>>>(r, dt);
   *launches += 1;
   return cudaGetLastError() == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }

@@ -19,7 +19,6 @@
 
 namespace eprem {
 
-constexpr int kSetupThreads = 64;  // small CTAs: FP64 latency bounds a node's chain
 
 // The instance for rows of P registers and V cells per access, or null.
 const void *node32_kernel_a(int P, int V);
@@ -27,9 +26,9 @@ const void *node32_kernel_b(int P, int V);
 
 // One thread per node: rates and sub-cycle counts (noderates.cuh) and the
 // coefficients rounded to float.
-__global__ void __launch_bounds__(kSetupThreads) k_node32_setup(RunView r) {
+__global__ void __launch_bounds__(128) k_node32_setup(RunView r) {
   const size_t SN = (size_t)r.S * r.N;
-  const size_t g = (size_t)blockIdx.x * kSetupThreads + threadIdx.x;
+  const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   int ns_f = 0, ns_c = 0;
   if (g < SN) {
     const int k = (int)(g % r.N);
@@ -86,7 +85,7 @@ int warps_held(int P) { return P <= 8 ? 8 : P <= 20 ? 5 : P <= 24 ? 4 : P <= 40 
 // 31 M instructions for each 32 rows and 13 E for each 32 columns (focusing at
 // a few sub-cycles).  More CTAs side by side on an SM overlap each other's
 // copies and barriers (one CTA alone takes twice the time, two half as much
-// again); a run with few nodes wants its CTAs spread over the SMs.  Measured, ms
+// again) and its own start (250); a run with few nodes wants its CTAs spread over the SMs.  Measured, ms
 // of 30 sub-steps: 96 streams x 1000 x 50 x 40, one node to a CTA 25.5, two 25.7,
 // three 26.9, five 30.9; 96 x 645 x 26 x 33, two 10.2, three 9.8, six 13.9; 24 x
 // 400 x 20 x 20, the choice 0.63, one 0.85, ten 0.84.
@@ -106,7 +105,7 @@ int plan_node32(int E, int M, size_t nodes, NodePlan *plan) {
     const double ctas = std::ceil((double)nodes / g);
     const int there = (int)std::min<double>(held, std::ceil(ctas / kSms));
     const double cost = (g * E + 31) / 32 * 31.0 * M + (g * M + 31) / 32 * 13.0 * E + 4.0 * E * M * g / 32;
-    const double time = std::ceil(ctas / (kSms * there)) * there * cost * (1.0 + 1.0 / there);
+    const double time = std::ceil(ctas / (kSms * there)) * there * (cost + 250.0) * (1.0 + 1.0 / there);
     if (best == 0.0 || time < 0.98 * best) {
       best = time;
       plan->nodes = g;
@@ -137,8 +136,8 @@ static int blocks_of(const RunView &r, int g) { return (int)(((size_t)r.S * r.N 
 
 int launch_node32_setup(const RunView &r, cudaStream_t st, uint64_t *launches) {
   const size_t SN = (size_t)r.S * r.N;
-  const unsigned blocks = (unsigned)((SN + kSetupThreads - 1) / kSetupThreads);
-  k_node32_setup<<<blocks, kSetupThreads, 0, st>>>(r);
+  const int t = node_threads(SN);
+  k_node32_setup<<<(unsigned)((SN + t - 1) / t), t, 0, st>>>(r);
   *launches += 1;
   return cudaGetLastError() == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }

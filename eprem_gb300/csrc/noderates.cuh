@@ -108,10 +108,26 @@ __device__ __forceinline__ NodeRates node_rates(const RunView &r, size_t g, int 
     // the speed is linear in a, so its maximum over the energies lies on the
     // rows of the smallest and largest a
     double amin = DBL_MAX, amax = -DBL_MAX;
-    for (int e = 0; e < r.E; e++) {
+    auto exact = [&](int e) {
       const double a = sub(mul(-r.ec[e].vgrid, o.dlnbds), mul(r.ec[e].two_vi, o.dupar));
       amin = a < amin ? a : amin;
       amax = a > amax ? a : amax;
+    };
+    // (1 / v is largest at the first energy, v below 1)
+    const double scale = fabs(o.dlnbds) + r.ec[0].two_vi * fabs(o.dupar);
+    if (float_scale(scale)) {
+      const float d = (float)o.dlnbds, u = 2.f * (float)o.dupar;
+      auto rough = [&](int e) { return -r.ec[e].v32 * d - r.ec[e].vi32 * u; };
+      float lo = FLT_MAX, hi = -FLT_MAX;
+      for (int e = 0; e < r.E; e++) {
+        lo = fminf(lo, rough(e));
+        hi = fmaxf(hi, rough(e));
+      }
+      const float near = 1e-4f * (float)scale;
+      for (int e = 0; e < r.E; e++)
+        if (rough(e) <= lo + near || rough(e) >= hi - near) exact(e);
+    } else {
+      for (int e = 0; e < r.E; e++) exact(e);
     }
     double vmax = 0.0;
     if (amin <= amax) vmax = fmax(focus_max(r, amin, o.b), focus_max(r, amax, o.b));

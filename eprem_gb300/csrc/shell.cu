@@ -591,11 +591,12 @@ int launch_perp_slice(const RunView &r, const int *shell_ent, int shell_L, const
 int launch_shell_coef(const RunView &r, const int *news, double kperxkpar, void *del,
                       cudaStream_t st, uint64_t *launches) {
   const size_t SN = (size_t)r.S * r.N;
-  const int blocks = (int)std::min<size_t>((SN + 127) / 128, 152 * 8);
+  const int t = node_threads(SN);
+  const int blocks = (int)std::min<size_t>((SN + t - 1) / t, 152 * 32);
   if (r.precision == EPREM_FP32)
-    k_shell_coef<float><<<blocks, 128, 0, st>>>(r, news, kperxkpar, (float *)del);
+    k_shell_coef<float><<<blocks, t, 0, st>>>(r, news, kperxkpar, (float *)del);
   else
-    k_shell_coef<double><<<blocks, 128, 0, st>>>(r, news, kperxkpar, (double *)del);
+    k_shell_coef<double><<<blocks, t, 0, st>>>(r, news, kperxkpar, (double *)del);
   ++*launches;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }
@@ -637,11 +638,12 @@ int launch_shell_diffuse(const RunView &r, const int *ent, int L, const void *de
 int launch_drift_coef(const RunView &r, const int *news, void *del, cudaStream_t st,
                       uint64_t *launches) {
   const size_t SN = (size_t)r.S * r.N;
-  const int blocks = (int)std::min<size_t>((SN + 127) / 128, 152 * 8);
+  const int t = node_threads(SN);
+  const int blocks = (int)std::min<size_t>((SN + t - 1) / t, 152 * 32);
   if (r.precision == EPREM_FP32)
-    k_drift_coef<float><<<blocks, 128, 0, st>>>(r, news, (float *)del);
+    k_drift_coef<float><<<blocks, t, 0, st>>>(r, news, (float *)del);
   else
-    k_drift_coef<double><<<blocks, 128, 0, st>>>(r, news, (double *)del);
+    k_drift_coef<double><<<blocks, t, 0, st>>>(r, news, (double *)del);
   ++*launches;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }
