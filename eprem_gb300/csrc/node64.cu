@@ -42,30 +42,49 @@ __device__ __forceinline__ int nan_or_inf(double v) {
   return isnan(v) ? EPREM_GPU_ERR_NAN : EPREM_GPU_ERR_INF;
 }
 
-// One pass of the focusing operator over a row: out_m = c0 f_m + c1 in_m
-// - c2 (q_{m+1} up_{m+1} - q_m up_m), up the upwind cell of `in`; walls at
-// both ends.  in and out may be the same row.  EULER: in = f, c0 + c1 = c2 = 1.
+// Cells whose loads are issued before any of their stores: a pass may write the
+// row that it reads, so the compiler keeps loads behind earlier stores, and a
+// cell at a time waits for shared memory each time.
+constexpr int kAhead = 4;
+
+// One pass of the focusing operator over a row: the Euler step of `in`, g_m = in_m
+// - (q_{m+1} up_{m+1} - q_m up_m) with up the upwind cell and walls at both ends,
+// then out_m = c0 f_m + c1 g_m (EULER: g_m).  in and out may be the same row.
 template <bool EULER>
 __device__ __forceinline__ void focus_pass(const double *f, const double *in, double *out,
-                                           const double *q, int M, double c0, double c1,
-                                           double c2) {
+                                           const double *q, int M, double c0, double c1) {
   double cur = in[0], qp = 0.0, up = 0.0;
-#pragma unroll 4
-  for (int m = 0; m + 1 < M; ++m) {
-    const double next = in[m + 1], qn = q[m + 1];
+  int m = 0;
+  for (; m + kAhead < M; m += kAhead) {
+    double x[kAhead], w[kAhead], o[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      x[j] = in[m + 1 + j];
+      w[j] = q[m + 1 + j];
+      o[j] = EULER ? 0.0 : f[m + j];
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const double un = negative(w[j]) ? x[j] : cur;
+      const double g = fma(qp, up, fma(-w[j], un, cur));
+      o[j] = EULER ? g : fma(c1, g, c0 * o[j]);
+      cur = x[j];
+      qp = w[j];
+      up = un;
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) out[m + j] = o[j];
+  }
+  for (; m < M; ++m) {
+    const bool wall = m + 1 == M;
+    const double next = wall ? cur : in[m + 1], qn = wall ? 0.0 : q[m + 1];
     const double un = negative(qn) ? next : cur;
-    if (EULER)
-      out[m] = fma(qp, up, fma(-qn, un, cur));
-    else
-      out[m] = fma(c0, f[m], fma(c1, cur, c2 * fma(qp, up, -(qn * un))));
+    const double g = fma(qp, up, fma(-qn, un, cur));
+    out[m] = EULER ? g : fma(c1, g, c0 * f[m]);
     cur = next;
     qp = qn;
     up = un;
   }
-  if (EULER)
-    out[M - 1] = fma(qp, up, cur);
-  else
-    out[M - 1] = fma(c0, f[M - 1], fma(c1, cur, c2 * (qp * up)));
 }
 
 // The same for the change operator on a column (stride `st`), with the seeds
@@ -73,32 +92,43 @@ __device__ __forceinline__ void focus_pass(const double *f, const double *in, do
 template <bool EULER>
 __device__ __forceinline__ void change_pass(const double *f, const double *in, double *out,
                                             const double *vw, int E, int st, double qa, double qb,
-                                            double b0, double b1, double c0, double c1, double c2) {
+                                            double b0, double b1, double c0, double c1) {
+  auto mix = [&](double fe, double g) { return EULER ? g : fma(c1, g, c0 * fe); };
   double cur = in[0], next = in[st];
   double q = fma(qa, vw[0], qb);
   double up = negative(q) ? next : cur;
-  auto put = [&](int e, double cur, double d) {  // d: minus the divergence
-    if (EULER)
-      out[e * st] = cur + d;
-    else
-      out[e * st] = fma(c0, f[e * st], fma(c1, cur, c2 * d));
-  };
-  // first energy: downwind from above, or the seed below
-  {
+  {  // first energy: downwind from above, or the seed below
     const double hi = negative(q) ? next : cur, lo = negative(q) ? cur : b0;
-    put(0, cur, -(q * (hi - lo)));
+    out[0] = mix(EULER ? 0.0 : f[0], fma(-q, hi - lo, cur));
   }
   double prev = cur;
   cur = next;
-#pragma unroll 4
-  for (int e = 1; e + 1 < E; ++e) {
+  int e = 1;
+  for (; e + kAhead < E; e += kAhead) {
+    double x[kAhead], w[kAhead], o[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      x[j] = in[(e + 1 + j) * st];
+      w[j] = fma(qa, vw[e + j], qb);
+      o[j] = EULER ? 0.0 : f[(e + j) * st];
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const double un = negative(w[j]) ? x[j] : cur;
+      o[j] = mix(o[j], fma(q, up, fma(-w[j], un, cur)));
+      prev = cur;
+      cur = x[j];
+      q = w[j];
+      up = un;
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) out[(e + j) * st] = o[j];
+  }
+  for (; e + 1 < E; ++e) {
     next = in[(e + 1) * st];
     const double qn = fma(qa, vw[e], qb);
     const double un = negative(qn) ? next : cur;
-    if (EULER)
-      out[e * st] = fma(q, up, fma(-qn, un, cur));
-    else
-      out[e * st] = fma(c0, f[e * st], fma(c1, cur, c2 * fma(q, up, -(qn * un))));
+    out[e * st] = mix(EULER ? 0.0 : f[e * st], fma(q, up, fma(-qn, un, cur)));
     prev = cur;
     cur = next;
     q = qn;
@@ -106,7 +136,7 @@ __device__ __forceinline__ void change_pass(const double *f, const double *in, d
   }
   // last energy: upwind from below, or the seed above
   const double hi = negative(q) ? b1 : cur, lo = negative(q) ? cur : prev;
-  put(E - 1, cur, -(q * (hi - lo)));
+  out[e * st] = mix(EULER ? 0.0 : f[e * st], fma(-q, hi - lo, cur));
 }
 
 __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) {
@@ -150,13 +180,13 @@ __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) 
 #pragma unroll 4
       for (int m = 1; m < M; ++m) q[m] = fma(a, g1[m], gb[m]);
       if (r.focus_alg == 1) {
-        for (int s = 0; s < c.ns_f; ++s) focus_pass<true>(row, row, row, q, M, 0.0, 1.0, 1.0);
+        for (int s = 0; s < c.ns_f; ++s) focus_pass<true>(row, row, row, q, M, 0.0, 1.0);
       } else {
         double *st = wk2 + (size_t)it * pitch;
         for (int s = 0; s < c.ns_f; ++s) {
-          focus_pass<true>(row, row, st, q, M, 0.0, 1.0, 1.0);
-          focus_pass<false>(row, st, st, q, M, 0.75, 0.25, 0.25);
-          focus_pass<false>(row, st, row, q, M, 1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0);
+          focus_pass<true>(row, row, st, q, M, 0.0, 1.0);
+          focus_pass<false>(row, st, st, q, M, 0.75, 0.25);
+          focus_pass<false>(row, st, row, q, M, 1.0 / 3.0, 2.0 / 3.0);
         }
       }
     }
@@ -193,14 +223,13 @@ __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) 
     const double qa = 0.5 * (c.step_c * c.cool) * am, qb = (c.step_c * c.cool) * bm;
     if (r.change_alg == 1) {
       for (int s = 0; s < c.ns_c; ++s)
-        change_pass<true>(col, col, col, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.0, 1.0, 1.0);
+        change_pass<true>(col, col, col, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.0, 1.0);
     } else {
       double *st = wk + (size_t)n * slab + m;
       for (int s = 0; s < c.ns_c; ++s) {
-        change_pass<true>(col, col, st, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.0, 1.0, 1.0);
-        change_pass<false>(col, st, st, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.75, 0.25, 0.25);
-        change_pass<false>(col, st, col, vw, E, pitch, qa, qb, c.bc0, c.bc1, 1.0 / 3.0, 2.0 / 3.0,
-                           2.0 / 3.0);
+        change_pass<true>(col, col, st, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.0, 1.0);
+        change_pass<false>(col, st, st, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.75, 0.25);
+        change_pass<false>(col, st, col, vw, E, pitch, qa, qb, c.bc0, c.bc1, 1.0 / 3.0, 2.0 / 3.0);
       }
     }
   }

@@ -197,6 +197,8 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
       dst[H] = FL;
       if (far) far[H] = FL;
     }
+    // what stays of the sum, formed while the rows travel
+    const double own = fma(-mR, FR, fma(-mL, FL, S));
     if (NC > 1)
       cluster.sync();
     else
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
       double Fin = __shfl_up_sync(FULL, FR, 1), Fout = __shfl_down_sync(FULL, FL, 1);
       if (lane == 0) Fin = my_hi[H];
       if (lane == 31) Fout = my_lo[H];
-      S = fma(mR, Fin - FR, fma(mL, Fout - FL, S));
+      S = fma(mR, Fin, fma(mL, Fout, own));
       const double b = S * omM;
       FL = FR = 0.0;
 #pragma unroll
