@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kNode32MaxThreads)
   // 1. rows in: where the pitch is M itself (V cells an odd number of times), in
   // the widest pieces that the CTA's place in f allows
   const int nval = rows * M;
-  const int place = (int)((g0 * E * M) & 3);
+  const int place = (int)(reinterpret_cast<uintptr_t>(fg) / sizeof(float) & 3);
   const bool flat = V != 4 && pitch == M && place != 1 && place != 3;
   if (flat) {
     if (place == 0) {

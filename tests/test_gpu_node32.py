@@ -62,3 +62,26 @@ def test_rows_with_a_far_tail(oracle_lib):
 
 def test_cooling_and_its_damping(oracle_lib):
     _check(W.custom(1, 2, 60, 12, 14, num_ep_steps=3, damp_cooling=0.5), oracle_lib)
+
+
+@pytest.mark.parametrize("nodes,mu", [(5, 33), (7, 22), (7, 20)])
+def test_parts_of_a_run_that_begin_anywhere_in_f(nodes, mu, oracle_lib):
+    """The host-memory update takes f's streams in parts: a part of odd streams
+    of nodes x 27 x mu cells begins at any of float's alignments.  Bit-identical
+    to the whole run's update."""
+    w = W.custom(4, 4, nodes, 27, mu, num_ep_steps=1)
+    _, g, f, values = primed_state(w, oracle_lib)
+    out = []
+    for host in (False, True):
+        run = EpremRun(w.dims(abi.EPREM_FP32), w.params, g)
+        run.upload_nodes(values)
+        if host:
+            got = np.empty_like(f)
+            run.update_energetic_particles_host(f, got, 0.0)
+        else:
+            run.upload_f(f)
+            run.update_energetic_particles(0.0)
+            got = run.download_f()
+        run.close()
+        out.append(got)
+    np.testing.assert_array_equal(out[0], out[1])
