@@ -120,7 +120,7 @@ extern "C" int eprem_gpu_plan_stream(int num_nodes, int num_mu, int m0, int prec
   StreamPlan p{};
   // (a run with few slabs may take a narrower shape)
   if (plan_stream(precision, num_nodes, num_mu, m0, variant, seed_boundary != 0,
-                  seed_boundary != 0, 1 << 20, &p))
+                  precision == EPREM_FP64 || seed_boundary != 0, 1 << 20, &p))
     return fail(EPREM_GPU_ERR_ARG, "no streaming kernel fits these sizes");
   const bool s2 = p.reg_coef == 2;
   const bool own = p.mirror && (num_mu == 20 || num_mu == 40);

@@ -150,12 +150,16 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
   const bool fast32 = dims->precision == EPREM_FP32 && params->adiabatic_focus_alg == 1 &&
                       params->adiabatic_change_alg == 1;
   const bool bc = params->use_ep_boundary > 0 && params->use_boundary_function > 0;
-  // the mirrored streaming kernel takes |mugrid| of a cell from its mirror cell
-  bool even_mu = true;
+  // the mirrored streaming kernels take |mugrid| of a cell from its mirror cell:
+  // in the FP64 form where the two differ by rounding alone
+  bool even_mu = true, mirror64 = true;
   for (int m = 0; m < M; m++)
     even_mu = even_mu && fabs(grids->mugrid[m] + grids->mugrid[M - 1 - m]) <= 1e-9 &&
               fabs(grids->mugrid[m] - grids->mugrid[0] - m * grids->dmu) <= 1e-9;
-  r->mirror_ok = bc && even_mu;
+  for (int m = 0; m < M; m++)
+    mirror64 = mirror64 && fabs(grids->mugrid[m] + grids->mugrid[M - 1 - m]) <= 4 * DBL_EPSILON &&
+               fabs(grids->mugrid[m]) <= (1.0 + 4 * DBL_EPSILON) * fabs(grids->mugrid[0]);
+  r->mirror_ok = dims->precision == EPREM_FP64 ? mirror64 : bc && even_mu;
   int prc = plan_stream(dims->precision, N, M, m0, params->stream_variant, bc, r->mirror_ok,
                         (long long)S * E, &r->splan);
   const bool fast64 = dims->precision == EPREM_FP64 && params->adiabatic_focus_alg <= 2 &&

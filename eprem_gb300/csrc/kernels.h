@@ -33,15 +33,15 @@ struct StreamPlan {
   int npt;       // stream2.cu: list nodes per thread
   int mirror;    // stream2m.cu (mmax is M itself there)
 };
-// bc: the run has the seed boundary (the mirrored kernel needs it); mirror_ok:
-// and a uniform symmetric mu grid; slabs: (stream, energy) slabs of a launch
+// bc: the run has the seed boundary (FP32's mirrored kernel needs it); mirror_ok:
+// FP32 form, and a uniform symmetric mu grid, FP64 form, a symmetric mu grid; slabs: (stream, energy) slabs of a launch
 int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool mirror_ok,
                 long long slabs, StreamPlan *plan);
 int launch_stream(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                   uint64_t *launches);
 int launch_seed_check(const RunView &r, cudaStream_t st, uint64_t *launches);
 // stream64.cu -- FP64 streaming in three operations per cell (plan.reg_coef == 3)
-bool stream64_shape(int N, int M, int m0, StreamPlan *plan);
+bool stream64_shape(int N, int M, int m0, bool mirror_ok, StreamPlan *plan);
 int launch_stream64(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                     uint64_t *launches);
 // stream2.cu -- FP32 streaming, several list nodes per thread (plan.reg_coef == 2)

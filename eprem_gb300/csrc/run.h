@@ -37,7 +37,7 @@ struct eprem_gpu_run {
   std::string skernel;  // eprem_gpu_stream_kernel's text
   eprem::NodePlan nplan{};
   int m0 = 0;
-  bool mirror_ok = false;  // seed boundary on, mu grid uniform and symmetric
+  bool mirror_ok = false;  // FP32: seed boundary on, mu grid uniform and symmetric; FP64: symmetric
   double norm_radius = 0, neg_beta = 0;
   double grid_dlnp = 0;  // dlnp of the momentum grid
   void *d_f = nullptr;

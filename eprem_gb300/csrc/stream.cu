@@ -14,9 +14,9 @@
 // The upwind coefficients mult*del_fac are fixed for the slab and held in
 // shared memory (the FP64 form is bound by the FP64 pipe, next to which
 // shared-memory loads cost nothing).  This is the plain FP64 form's kernel for
-// streams too long for stream64.cu, which takes three FP64 operations per cell
-// and sub-cycle where this one takes four but twice the shared memory; the
-// FP32 form streams with stream2.cu.
+// mu grids whose cells do not mirror each other and for streams too long for
+// stream64.cu, which takes three FP64 operations per cell and sub-cycle where
+// this one takes four; the FP32 form streams with stream2m.cu and stream2.cu.
 // seedPopulationCheck (src/energeticParticlesBoundary.c:28-59) is applied as
 // the slab is loaded; thinned-out nodes receive their reference node's values
 // on write-back, as the reference's shellRef copy does (:2448-2455).
@@ -280,9 +280,9 @@ static int threads_for(int mmax) {
 // streams x 50 E, ms of streaming in 30 sub-steps, stream2.cu's automatic
 // choice against it: M = 28, N = 1000 291 and 163; M = 33, N = 645, 26 E 179
 // and 59; M = 8, N = 1000 83 and 52; M = 64, N = 500 117 and 116.
-// The FP64 form has one kernel per stream length (stream64.cu, or
-// k_stream where a cluster of that one cannot hold the stream); variants 1 and
-// 2 name it there.
+// The FP64 form has one kernel per stream length and mu grid (stream64.cu, or
+// k_stream where a cluster of that one cannot hold the stream, or the cells of
+// the mu grid do not mirror each other); variants 1 and 2 name it there.
 int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool mirror_ok,
                 long long slabs, StreamPlan *plan) {
   if (precision == EPREM_FP32) {
@@ -302,7 +302,7 @@ int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool 
     return EPREM_GPU_ERR_ARG;
   }
   if (variant > 2) return EPREM_GPU_ERR_ARG;
-  if (stream64_shape(N, M, m0, plan)) return 0;
+  if (stream64_shape(N, M, m0, mirror_ok, plan)) return 0;
   int mmax = 0;
   for (int b : kStreamBins)
     if (M <= b) { mmax = b; break; }

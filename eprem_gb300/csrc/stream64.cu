@@ -17,16 +17,27 @@
 // two fused multiply-adds, and one more for the new F.  For a node's particle
 // number to be kept over 1e5 sub-cycles A_j + C_j must be em exactly: C_j is
 // rounded to a multiple of em's last place, which makes the difference exact.
-// S is summed afresh from the cells at every launch.
-// Coefficients {A, C} sit in shared memory ([cell][thread], one 16-byte load
-// per cell); padding cells of a half have A = C = |mu| = 0 and touch nothing.
+// b itself is carried, not S (b' = b + (1 - em) / M m (F_up - F)), and F in units
+// of the largest |mu|, mu_0's, whose cell then enters without an operation; b is
+// formed afresh from the cells at every launch.
+//
+// The mu grid's cells mirror each other, so cell j and cell M - 1 - j share one
+// {A, C}: 16 bytes of shared memory per slot and thread ([slot][thread], one
+// load).  A half without an upwind node (the first list node's mu >= 0 cells,
+// the last one's mu < 0 cells) takes its own cells as the upwind ones instead of
+// a C of its own.  Padding cells have C = |mu| = 0; what they hold goes nowhere.
 //
 // Measured on a GB300, per launch, against the four-operation kernel of
 // stream.cu with its fixed CTA widths: 6 streams x 1000 x 50 x 40, 17.9 ->
-// 13.9 ms (four CTAs of 256 threads per slab; 75 % of the FP64 FMA peak, the
-// rest being barriers and the last slabs); 24 x 400 x 20 x 20, 1.53 -> 0.97
-// ms; 24 x 60 x 12 x 6 with 13,000 sub-cycles, 12.9 -> 1.83 ms (64 threads
-// where the fixed width was 1024; latency of the chain of one sub-cycle).
+// 12.3 ms (two CTAs of 512 threads per slab; 85 % of the FP64 FMA peak; with
+// {A, C} per cell instead, four CTAs of 256 threads, 13.9 ms: clusters of four
+// leave 8 of the 152 SMs without work, and 8 warps do not cover the loads);
+// 24 x 400 x 20 x 20, 1.53 -> 0.90 ms (13 warps, so one scheduler of an SM has
+// four of them and the others three: the rest of the peak); 24 x 60 x 12 x 6
+// with 13,000 sub-cycles, 12.9 -> 1.44 ms (64 threads where the fixed width was
+// 1024; latency of the chain of one sub-cycle).  The FP64 pipe takes a warp's
+// FMA in 64 cycles of its scheduler however independent, an addition or a
+// product alone in 76.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -36,16 +47,18 @@ namespace cg = cooperative_groups;
 
 namespace eprem {
 
-// Slots per direction of mu, and the most threads of a CTA: {A, C} of 2 H
-// cells take 32 H bytes of shared memory per thread, f 4 H registers.
-#define EPREM_S64_BINS(X)                                                              \
-  X(3, 2, 512) X(4, 3, 512) X(5, 4, 512) X(6, 5, 512) X(8, 6, 512) X(10, 8, 512)       \
-  X(12, 10, 384) X(14, 12, 384) X(16, 14, 384) X(20, 16, 256) X(24, 20, 256) X(32, 24, 192)
+// Slots per direction of mu, how many are always in use, and the most threads
+// of a CTA: f takes 4 H registers, {A, C} 16 H bytes of shared memory per
+// thread.  Whole warps per scheduler: its quarter of the register file goes to
+// the warps that it is given, so 13 warps have no more registers than 16.
+#define EPREM_S64_BINS(X)                                                             \
+  X(3, 2, 512) X(4, 3, 512) X(5, 4, 512) X(6, 5, 512) X(8, 6, 512) X(10, 8, 512)      \
+  X(12, 10, 512) X(14, 12, 512) X(16, 14, 512) X(20, 16, 512) X(24, 20, 384) X(32, 24, 256)
 
 template <int H>
 constexpr size_t stream64_smem(int threads) {
-  return sizeof(double2) * 2 * H * threads + sizeof(double) * 2 * 2 * (threads / 32 + 1) * (H + 1) +
-         sizeof(double) * 2 * H;
+  return sizeof(double2) * H * threads + sizeof(double) * 2 * 2 * (threads / 32 + 1) * (H + 1) +
+         sizeof(double) * (H + 9);
 }
 
 // x (0 <= x < em) to the nearest multiple of em's last place, so that em - x
@@ -58,6 +71,18 @@ __device__ __forceinline__ double to_place_of(double em, double x) {
   return __dsub_rn(__dadd_rn(x, k), k);
 }
 
+// the shared memory of CTA `rank` of the cluster at this CTA's `p`, and a store there
+__device__ __forceinline__ uint32_t remote(const double *p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(a)
+      : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void store_remote(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
 // H slots per direction, of which the first HLO are always in use.
 template <int H, int HLO, int TMAX>
 __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
@@ -65,11 +90,12 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
   constexpr int HP = H + 1;  // a halo row: the half's cells, then its F
   extern __shared__ __align__(16) unsigned char sm64[];
   const int T = blockDim.x, W = T >> 5;
-  double2 *tab = reinterpret_cast<double2 *>(sm64);  // [2 H][T] {A, C}: mu < 0 slots, mu >= 0 slots
+  double2 *tab = reinterpret_cast<double2 *>(sm64);  // [H][T] {A, C} of both cells of a slot
   // halo rows by sub-cycle parity p: hi(p, w), the row of the thread before
   // warp w (mu >= 0); lo(p, w), the row of warp w's first thread (mu < 0)
-  double *halo = reinterpret_cast<double *>(tab + 2 * H * T);
-  double *amu = halo + 2 * 2 * (W + 1) * HP;  // [2 H] |mugrid|
+  double *halo = reinterpret_cast<double *>(tab + H * T);
+  double *rho = halo + 2 * 2 * (W + 1) * HP;  // [H] |mu| over its largest
+  double *bc = rho + H;  // [3][3] of the boundary's nodes: a cell, b, F
   auto hi = [&](int p, int w) { return halo + ((p * 2 + 0) * (W + 1) + w) * HP; };
   auto lo = [&](int p, int w) { return halo + ((p * 2 + 1) * (W + 1) + w) * HP; };
 
@@ -99,68 +125,65 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
     atomicAdd(&r.status->stream_cs, (unsigned long long)nsteps * L * M);
   }
   for (int j = tid; j < 2 * 2 * (W + 1) * HP; j += T) halo[j] = 0.0;
-  for (int j = tid; j < 2 * H; j += T) {
-    const int h = j < H ? j : j - H;
-    const bool in = j < H ? h < nL : h < nR;
-    amu[j] = in ? fabs(r.mugrid[j < H ? h : m0 + h]) : 0.0;
-  }
+  const double mu0 = fabs(r.mugrid[0]);
+  for (int j = tid; j < H; j += T) rho[j] = j < nL ? fabs(r.mugrid[j]) / mu0 : 0.0;
   __syncthreads();
 
   const int i = crank * T + tid;
-  const bool active = i < L;
+  const bool active = i < L, first = i == 0, last = i == L - 1;
   const bool warp_live = crank * T + (warp << 5) < L;
   const size_t sN = (size_t)s * N;
   double fL[H], fR[H];
-  double S = 0.0, FL = 0.0, FR = 0.0;
-  double mL = 0.0, mR = 0.0, omM = 0.0, bcv = 0.0, em = 0.0;
-  bool bc_node = false;
-  int k = 0;
+  double b = 0.0, FL = 0.0, FR = 0.0;
+  double m = 0.0, omM = 0.0, em = 0.0;
+  const bool bc_node = r.use_bc && i < 3;
   const double *row = nullptr;
-  double seedv = 0.0, mult = 0.0;
+  double seedv = 0.0;
   if (active) {
-    k = r.list[sN + i];
-    const size_t g = sN + k;
+    const size_t g = sN + r.list[sN + i];
     const double tau = ec.vgrid_i * (ec.rig_lamo * r.mfp_node[g]);
     const double dsi = r.ds_i[sN + i];
-    mult = (dtProp > tau) ? dsi * tau * dtProp_i : dsi * 1.0;
+    const double mult = (dtProp > tau) ? dsi * tau * dtProp_i : dsi * 1.0;
     em = r.relax_in_stream ? exp(-dtProp / tau) : 1.0;
     omM = (1.0 - em) * (1.0 / M);
     seedv = seed_value(r, ec, r.seed_radial[g]);
     row = reinterpret_cast<const double *>(r.f) + (g * r.E + e) * M;
-    // the first list node keeps its mu >= 0 cells (src/energeticParticles.c:
-    // 2381), the last its mu < 0 cells (:2393)
-    const double vdt = ec.vgrid * dtProp;
-    mR = i == 0 ? 0.0 : mult * vdt;
-    mL = i == L - 1 ? 0.0 : mult * vdt;
-    bc_node = r.use_bc && i < 3;
-    bcv = seedv;
+    m = mult * (ec.vgrid * dtProp);
   }
-  double sumL = 0.0, sumR = 0.0;  // of |mu|
+  double S = 0.0, sum = 0.0;  // sum: of rho
 #pragma unroll
   for (int j = 0; j < H; ++j) {
-    sumL += amu[j];
-    sumR += amu[H + j];
+    sum += rho[j];
+    // few rows' loads in flight at a time: all of them together would spill
+    if (j % 4 == 0) asm volatile("" ::: "memory");
     fL[j] = fR[j] = 0.0;
-    double cl = 0.0, cr = 0.0;
+    double c = 0.0;
     if (active && j < nL) {
       const double v = row[j];
       fL[j] = (r.check_seed && v < seedv) ? seedv : v;
-      cl = to_place_of(em, em * (mL * amu[j]));
+      c = to_place_of(em, em * (m * (rho[j] * mu0)));
     }
     if (active && j < nR) {
-      const double v = row[m0 + j];
+      const double v = row[M - 1 - j];
       fR[j] = (r.check_seed && v < seedv) ? seedv : v;
-      cr = to_place_of(em, em * (mR * amu[H + j]));
     }
-    tab[j * T + tid] = make_double2(active && j < nL ? em - cl : 0.0, cl);
-    tab[(H + j) * T + tid] = make_double2(active && j < nR ? em - cr : 0.0, cr);
+    tab[j * T + tid] = make_double2(active && j < nmax ? em - c : 0.0, c);
     S += fL[j] + fR[j];
-    FL = fma(amu[j], fL[j], FL);
-    FR = fma(amu[H + j], fR[j], FR);
+    FL = fma(rho[j], fL[j], FL);
+    FR = fma(rho[j], fR[j], FR);
   }
-  // halo rows this CTA fills in its neighbours
-  double *next_hi = (NC > 1 && crank < NC - 1) ? cluster.map_shared_rank(halo, crank + 1) : nullptr;
-  double *prev_lo = (NC > 1 && crank > 0) ? cluster.map_shared_rank(halo, crank - 1) : nullptr;
+  b = S * omM;
+  if (bc_node) {
+    bc[3 * i] = seedv;
+    bc[3 * i + 1] = M * seedv * omM;
+    bc[3 * i + 2] = sum * seedv;
+  }
+  // the first list node keeps its mu >= 0 cells (src/energeticParticles.c:
+  // 2381), the last its mu < 0 cells (:2393): both are their own upwind node
+  const double gm = m * mu0 * omM;
+  const int from_in = first || lane == 0 ? lane : lane - 1;
+  const int from_out = last || lane == 31 ? lane : lane + 1;
+  const bool row_in = lane == 0 && !first, row_out = lane == 31 && !last;
   if (NC > 1)
     cluster.sync();  // halo zeroing is complete before any remote store lands
   else
@@ -170,76 +193,77 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
     const int p = step & 1;
     if (bc_node) {  // the seed boundary (:2361-2370)
 #pragma unroll
-      for (int j = 0; j < H; ++j) fL[j] = fR[j] = bcv;
-      S = M * bcv;
-      FL = sumL * bcv;
-      FR = sumR * bcv;
+      for (int j = 0; j < H; ++j) fL[j] = fR[j] = bc[3 * i];
+      b = bc[3 * i + 1];
+      FL = FR = bc[3 * i + 2];
     }
     if (lane == 31 && warp_live) {
       double *dst = hi(p, warp + 1);
-      double *far = (warp == W - 1 && next_hi) ? next_hi + ((p * 2 + 0) * (W + 1)) * HP : nullptr;
 #pragma unroll
-      for (int j = 0; j < H; ++j) {
-        dst[j] = fR[j];
-        if (far) far[j] = fR[j];
-      }
+      for (int j = 0; j < H; ++j) dst[j] = fR[j];
       dst[H] = FR;
-      if (far) far[H] = FR;
+      if (warp == W - 1 && crank < NC - 1) {
+        const uint32_t far = remote(hi(p, 0), crank + 1);
+#pragma unroll
+        for (int j = 0; j < H; ++j) store_remote(far + 8 * j, fR[j]);
+        store_remote(far + 8 * H, FR);
+      }
     }
     if (lane == 0 && warp_live) {
       double *dst = lo(p, warp);
-      double *far = (warp == 0 && prev_lo) ? prev_lo + ((p * 2 + 1) * (W + 1) + W) * HP : nullptr;
 #pragma unroll
-      for (int j = 0; j < H; ++j) {
-        dst[j] = fL[j];
-        if (far) far[j] = fL[j];
-      }
+      for (int j = 0; j < H; ++j) dst[j] = fL[j];
       dst[H] = FL;
-      if (far) far[H] = FL;
+      if (warp == 0 && crank > 0) {
+        const uint32_t far = remote(lo(p, W), crank - 1);
+#pragma unroll
+        for (int j = 0; j < H; ++j) store_remote(far + 8 * j, fL[j]);
+        store_remote(far + 8 * H, FL);
+      }
     }
     // what stays of the sum, formed while the rows travel
-    const double own = fma(-mR, FR, fma(-mL, FL, S));
+    b = fma(-gm, FR, fma(-gm, FL, b));
     if (NC > 1)
       cluster.sync();
     else
       __syncthreads();
     if (warp_live) {
       const double *my_hi = hi(p, warp), *my_lo = lo(p, warp + 1);
-      double Fin = __shfl_up_sync(FULL, FR, 1), Fout = __shfl_down_sync(FULL, FL, 1);
-      if (lane == 0) Fin = my_hi[H];
-      if (lane == 31) Fout = my_lo[H];
-      S = fma(mR, Fin, fma(mL, Fout, own));
-      const double b = S * omM;
-      FL = FR = 0.0;
+      double Fin = __shfl_sync(FULL, FR, from_in), Fout = __shfl_sync(FULL, FL, from_out);
+      if (row_in) Fin = my_hi[H];
+      if (row_out) Fout = my_lo[H];
+      b = fma(gm, Fin, fma(gm, Fout, b));
 #pragma unroll
       for (int j = 0; j < H; ++j) {
         if (j < HLO || j < nmax) {
-          double nl = __shfl_down_sync(FULL, fL[j], 1), nr = __shfl_up_sync(FULL, fR[j], 1);
-          if (lane == 31) nl = my_lo[j];
-          if (lane == 0) nr = my_hi[j];
-          const double2 al = tab[j * T + tid], ar = tab[(H + j) * T + tid];
-          fL[j] = fma(al.x, fL[j], fma(al.y, nl, b));
-          fR[j] = fma(ar.x, fR[j], fma(ar.y, nr, b));
-          FL = fma(amu[j], fL[j], FL);
-          FR = fma(amu[H + j], fR[j], FR);
+          double nl = __shfl_sync(FULL, fL[j], from_out), nr = __shfl_sync(FULL, fR[j], from_in);
+          if (row_out) nl = my_lo[j];
+          if (row_in) nr = my_hi[j];
+          const double2 a = tab[j * T + tid];
+          fL[j] = fma(a.x, fL[j], fma(a.y, nl, b));
+          fR[j] = fma(a.x, fR[j], fma(a.y, nr, b));
+          FL = j ? fma(rho[j], fL[j], FL) : fL[0];
+          FR = j ? fma(rho[j], fR[j], FR) : fR[0];
         }
       }
     }
   }
 
   if (active) {
-    int code = 0;
+    int code = 0, bad = 0, mu = 0;  // the first value that is not a number or infinite
+    const int k = r.list[sN + i];
 #pragma unroll
     for (int j = 0; j < H; ++j) {
       if (j < nL) {
-        if (bad_value(fL[j], &code)) set_error(r, code, 1, s, k, e, j);
+        if (bad_value(fL[j], &code) && !bad) bad = code, mu = j;
         fL[j] = fL[j] < DBL_MIN ? DBL_MIN : fL[j];
       }
       if (j < nR) {
-        if (bad_value(fR[j], &code)) set_error(r, code, 1, s, k, e, m0 + j);
+        if (bad_value(fR[j], &code) && !bad) bad = code, mu = M - 1 - j;
         fR[j] = fR[j] < DBL_MIN ? DBL_MIN : fR[j];
       }
     }
+    if (bad) set_error(r, bad, 1, s, k, e, mu);
     // node k and the thinned nodes that reference it (previous list node + 1 .. k)
     const int kfirst = (i == 0) ? 0 : r.list[sN + i - 1] + 1;
     for (int kk = kfirst; kk <= k; ++kk) {
@@ -247,7 +271,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
 #pragma unroll
       for (int j = 0; j < H; ++j) {
         if (j < nL) op[j] = fL[j];
-        if (j < nR) op[m0 + j] = fR[j];
+        if (j < nR) op[M - 1 - j] = fR[j];
       }
     }
   }
@@ -257,12 +281,14 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
 // The CTA and cluster of a run: the fewest CTAs that hold a stream of N
 // nodes, of equal width in whole warps, so that no idle warp takes part in the
 // barriers.  Splitting a slab further does not pay (per launch, 24 x 400 x 20
-// x 20: one CTA 0.97 ms, two 1.02, four 1.15, seven 1.00; 6 x 1000 x 50 x 40:
-// four 13.95, eight 13.73): the FP64 pipe is the bound and a cluster's barrier
-// costs more than a CTA's.  False where a half of mu has more than 32 cells or
-// a portable cluster (8 CTAs) cannot hold the stream; those streams keep the
-// kernel of stream.cu, whose coefficients need half the shared memory.
-bool stream64_shape(int N, int M, int m0, StreamPlan *plan) {
+// x 20: one CTA 0.90 ms, two 0.91, three or four resident CTAs of fewer
+// registers 0.94 to 0.98; 6 x 1000 x 50 x 40: two 12.3 ms, three 14.1, four
+// 13.3): the FP64 pipe is the bound and a cluster's barrier costs more than a
+// CTA's.  False where the mu grid does not mirror, a half of mu has more than 32
+// cells or a portable cluster (8 CTAs) cannot hold the stream; those runs keep
+// the kernel of stream.cu, which takes any mu grid and longer streams.
+bool stream64_shape(int N, int M, int m0, bool mirror_ok, StreamPlan *plan) {
+  if (!mirror_ok || m0 < 1 || (2 * m0 != M && 2 * m0 != M - 1 && 2 * m0 != M + 1)) return false;
   const int n = m0 > M - m0 ? m0 : M - m0;
   int h = 0, tmax = 0;
 #define EPREM_S64_PICK(HH, LO, TT) \

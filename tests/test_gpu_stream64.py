@@ -1,6 +1,6 @@
 """FP64 streaming in three operations per cell (stream64.cu): list lengths at
 the edges of warps, CTAs and clusters, mu counts at the edges of its bins,
-uneven splits of mu, and streams long enough to fall back to the four-operation
+mu grids that do not mirror, and streams long enough to fall back to the four-operation
 kernel, each within the plain form's 1e-12 of the oracle on every cell."""
 import numpy as np
 import pytest
@@ -52,12 +52,18 @@ def test_switches(seed_check, boundary, oracle_lib):
            oracle_lib)
 
 
+@pytest.mark.parametrize("nodes,mu", [(512, 6), (512, 12), (512, 20), (512, 32), (512, 39),
+                                      (384, 47), (256, 63), (257, 64)])
+def test_widest_block_of_a_bin(nodes, mu, oracle_lib):
+    assert _check(_streaming(nodes, mu), oracle_lib).startswith("k_stream64")
+
+
 @pytest.mark.parametrize("m0", [0, 2, 7, 10])
-def test_uneven_split_of_mu(m0, oracle_lib):
+def test_mu_grid_that_does_not_mirror(m0, oracle_lib):
     w = _streaming(60, 10)
     g = W.build_grids(w)
     g["mugrid"] = (np.arange(10) - m0 + 0.5) / 11.0
-    _check(w, oracle_lib, g)
+    assert _check(w, oracle_lib, g).startswith("k_stream<")
 
 
 def test_thinned_stream(oracle_lib):
@@ -71,9 +77,11 @@ def test_strong_scattering(oracle_lib):
     _check(_streaming(60, 8, lamo=1e-4), oracle_lib)
 
 
-@pytest.mark.parametrize("nodes,kernel", [(2048, "k_stream64<40>"), (2049, "k_stream<40>")])
-def test_longest_streams(nodes, kernel, oracle_lib):
-    w = W.custom(1, 1, nodes, 2, 40, e_max=0.2, num_ep_steps=1, use_adiabatic_focus=0,
+@pytest.mark.parametrize("nodes,mu,kernel", [(4096, 8, "k_stream64<8>"), (4097, 8, "k_stream<8>"),
+                                             (3072, 48, "k_stream64<48>"),
+                                             (2049, 64, "k_stream<64>")])
+def test_longest_streams(nodes, mu, kernel, oracle_lib):
+    w = W.custom(1, 1, nodes, 2, mu, e_max=0.2, num_ep_steps=1, use_adiabatic_focus=0,
                  use_adiabatic_change=0)
     assert _check(w, oracle_lib).startswith(kernel)
 
