@@ -138,7 +138,9 @@ extern "C" const char *eprem_gpu_stream_kernel(eprem_gpu_run *r) {
   const StreamPlan &p = r->splan;
   char buf[96];
   if (p.reg_coef != 2)
-    snprintf(buf, sizeof(buf), "%s<%d> cluster %d", p.reg_coef == 3 ? "k_stream64" : "k_stream",
+    snprintf(buf, sizeof(buf), "%s<%d> cluster %d", p.reg_coef == 4   ? "k_stream64_short"
+             : p.reg_coef == 3 ? "k_stream64"
+                               : "k_stream",
              p.mmax, p.cluster);
   else
     snprintf(buf, sizeof(buf), "%s<%d,%d,%d> cluster %d",

@@ -27,7 +27,7 @@ struct StreamPlan {
   int threads;   // threads per CTA
   int cluster;   // CTAs per (stream, energy) slab
   int reg_coef;  // coefficients in registers (1), shared memory (0); 2: stream2.cu;
-                 // 3: stream64.cu
+                 // 3: stream64.cu, 4: its kernel for short streams
   int packed;    // stream2.cu: fp32x2 arithmetic on pairs of mu cells
   int filled;    // stream2.cu: M fills the bin, m0 = M/2 (guards known at compile time)
   int npt;       // stream2.cu: list nodes per thread
@@ -40,8 +40,8 @@ int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool 
 int launch_stream(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                   uint64_t *launches);
 int launch_seed_check(const RunView &r, cudaStream_t st, uint64_t *launches);
-// stream64.cu -- FP64 streaming in three operations per cell (plan.reg_coef == 3)
-bool stream64_shape(int N, int M, int m0, bool mirror_ok, StreamPlan *plan);
+// stream64.cu -- FP64 streaming in three operations per cell (plan.reg_coef 3 and 4)
+bool stream64_shape(int N, int M, int m0, bool mirror_ok, long long slabs, StreamPlan *plan);
 int launch_stream64(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                     uint64_t *launches);
 // stream2.cu -- FP32 streaming, several list nodes per thread (plan.reg_coef == 2)

@@ -302,7 +302,7 @@ int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool 
     return EPREM_GPU_ERR_ARG;
   }
   if (variant > 2) return EPREM_GPU_ERR_ARG;
-  if (stream64_shape(N, M, m0, mirror_ok, plan)) return 0;
+  if (stream64_shape(N, M, m0, mirror_ok, slabs, plan)) return 0;
   int mmax = 0;
   for (int b : kStreamBins)
     if (M <= b) { mmax = b; break; }
@@ -357,7 +357,7 @@ int launch_stream(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t
                   uint64_t *launches) {
   if (plan.reg_coef == 2) return launch_stream2(r, plan, m0, st, launches);
   if (r.precision != EPREM_FP64) return EPREM_GPU_ERR_ARG;
-  if (plan.reg_coef == 3) return launch_stream64(r, plan, m0, st, launches);
+  if (plan.reg_coef >= 3) return launch_stream64(r, plan, m0, st, launches);
   const cudaError_t err = dispatch_mmax<double, false>(r, plan, m0, st);
   *launches += 1;
   return err == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;

@@ -34,8 +34,8 @@
 // leave 8 of the 152 SMs without work, and 8 warps do not cover the loads);
 // 24 x 400 x 20 x 20, 1.53 -> 0.90 ms (13 warps, so one scheduler of an SM has
 // four of them and the others three: the rest of the peak); 24 x 60 x 12 x 6
-// with 13,000 sub-cycles, 12.9 -> 1.44 ms (64 threads where the fixed width was
-// 1024; latency of the chain of one sub-cycle).  The FP64 pipe takes a warp's
+// with 13,000 sub-cycles, 12.9 -> 0.91 ms (k_stream64_short on 128 threads where
+// the fixed width was 1024; latency of the chain of one sub-cycle).  The FP64 pipe takes a warp's
 // FMA in 64 cycles of its scheduler however independent, an addition or a
 // product alone in 76.
 #include <cooperative_groups.h>
@@ -54,6 +54,14 @@ namespace eprem {
 #define EPREM_S64_BINS(X)                                                             \
   X(3, 2, 512) X(4, 3, 512) X(5, 4, 512) X(6, 5, 512) X(8, 6, 512) X(10, 8, 512)      \
   X(12, 10, 512) X(14, 12, 512) X(16, 14, 512) X(20, 16, 512) X(24, 20, 384) X(32, 24, 256)
+
+constexpr int kS64ShortNodes = 128;
+
+template <int H>
+constexpr size_t stream64_short_smem(int nodes) {
+  return sizeof(double2) * H * nodes +
+         sizeof(double) * (2 * 2 * (nodes / 32 * H + nodes) + H + 9);
+}
 
 template <int H>
 constexpr size_t stream64_smem(int threads) {
@@ -278,6 +286,176 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
   if (NC > 1) cluster.sync();  // no CTA leaves while a neighbour may still store into it
 }
 
+// The same for streams of at most kS64ShortNodes nodes in launches that leave an
+// SM's schedulers with little to do: a warp's FP64 operations follow one another
+// at 64 cycles each there, so the directions of mu go to a thread each, which has
+// half of them (both form b, from the moments in shared memory: 6 H + 6
+// operations per node where the other kernel takes 6 H + 2).  24 streams x 60 x
+// 12 x 6 with 13,000 sub-cycles, per launch: 1.44 -> 0.91 ms.
+template <int H, int HLO>
+__global__ void __launch_bounds__(2 * kS64ShortNodes, 1) k_stream64_short(RunView r, int m0) {
+  constexpr unsigned FULL = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char sm64[];
+  const int T = blockDim.x >> 1, W = T >> 5;  // nodes, and warps per direction of mu
+  double2 *tab = reinterpret_cast<double2 *>(sm64);  // [H][T] {A, C} of both cells of a slot
+  // the rows of cells at the warps' edges, by sub-cycle parity p and direction
+  // d: in(p, 0, w) that of the thread after warp w (mu < 0), in(p, 1, w) that of
+  // the thread before it (mu >= 0)
+  double *halo = reinterpret_cast<double *>(tab + H * T);
+  double *Fs = halo + 2 * 2 * W * H;  // [2][2][T] F
+  double *rho = Fs + 2 * 2 * T;       // [H] |mu| over its largest
+  double *bc = rho + H;               // [3][3] of the boundary's nodes: a cell, b, F
+  auto in = [&](int p, int d, int w) { return halo + ((p * 2 + d) * W + w) * H; };
+  auto mom = [&](int p, int d, int t) { return Fs + (p * 2 + d) * T + t; };
+
+  const int s = blockIdx.y;
+  const int e = r.E - 1 - (int)blockIdx.z;  // most sub-cycles first
+  const int lane = threadIdx.x & 31;
+  const int d = (int)threadIdx.x >= T;  // 0: the node's mu < 0 cells, 1: its mu >= 0 cells
+  const int tid = threadIdx.x - (d ? T : 0), warp = tid >> 5;
+  const int M = r.M, N = r.N;
+  const int nL = m0, nR = M - m0, nmax = nL > nR ? nL : nR, nd = d ? nR : nL;
+  const int L = r.list_size[s];
+  if (L < 3) return;  // flagged by the geometry pass
+
+  const EnergyConsts ec = r.ec[e];
+  const double dtMin = 0.4 * r.ds_min[s] * ec.vgrid_i;
+  const double nst = floor(r.dt / dtMin + 1.0);
+  if (!(nst <= (double)r.max_subcycles)) {
+    if (threadIdx.x == 0) set_error(r, EPREM_GPU_ERR_SUBCYCLES, 1, s, -1, e, -1);
+    return;
+  }
+  const int nsteps = (int)nst;
+  const double dtProp = r.dt / (1.0 * nsteps);
+  const double dtProp_i = 1.0 / dtProp;
+  if (threadIdx.x == 0) {
+    atomicMax(&r.status->max_stream, nsteps);
+    atomicAdd(&r.status->stream_cs, (unsigned long long)nsteps * L * M);
+  }
+  for (int j = threadIdx.x; j < 2 * 2 * (W * H + T); j += 2 * T) halo[j] = 0.0;
+  const double mu0 = fabs(r.mugrid[0]);
+  for (int j = threadIdx.x; j < H; j += 2 * T) rho[j] = j < nL ? fabs(r.mugrid[j]) / mu0 : 0.0;
+  __syncthreads();
+
+  const int i = tid;
+  const bool active = i < L, first = i == 0, last = i == L - 1;
+  const bool warp_live = (warp << 5) < L;
+  const size_t sN = (size_t)s * N;
+  double f[H];
+  double b = 0.0, F = 0.0;
+  double m = 0.0, omM = 0.0, em = 0.0;
+  const bool bc_node = r.use_bc && i < 3;
+  const double *row = nullptr;
+  const int at = d ? M - 1 : 0, sg = d ? -1 : 1;  // slot j: cell at + sg j
+  double seedv = 0.0;
+  if (active) {
+    const size_t g = sN + r.list[sN + i];
+    const double tau = ec.vgrid_i * (ec.rig_lamo * r.mfp_node[g]);
+    const double dsi = r.ds_i[sN + i];
+    const double mult = (dtProp > tau) ? dsi * tau * dtProp_i : dsi * 1.0;
+    em = r.relax_in_stream ? exp(-dtProp / tau) : 1.0;
+    omM = (1.0 - em) * (1.0 / M);
+    seedv = seed_value(r, ec, r.seed_radial[g]);
+    row = reinterpret_cast<const double *>(r.f) + (g * r.E + e) * M + at;
+    m = mult * (ec.vgrid * dtProp);
+  }
+  double S = 0.0, sum = 0.0;  // sum: of rho
+#pragma unroll
+  for (int j = 0; j < H; ++j) {
+    sum += rho[j];
+    // few rows' loads in flight at a time: all of them together would spill
+    if (j % 4 == 0) asm volatile("" ::: "memory");
+    f[j] = 0.0;
+    if (active && j < nd) {
+      const double v = row[sg * j];
+      f[j] = (r.check_seed && v < seedv) ? seedv : v;
+    }
+    if (!d) {
+      const double c = active && j < nL ? to_place_of(em, em * (m * (rho[j] * mu0))) : 0.0;
+      tab[j * T + tid] = make_double2(active && j < nmax ? em - c : 0.0, c);
+    }
+    S += f[j];
+    F = fma(rho[j], f[j], F);
+  }
+  if (active) *mom(0, d, tid) = S;
+  if (bc_node && !d) {
+    bc[3 * i] = seedv;
+    bc[3 * i + 1] = M * seedv * omM;
+    bc[3 * i + 2] = sum * seedv;
+  }
+  // the first list node keeps its mu >= 0 cells (src/energeticParticles.c:
+  // 2381), the last its mu < 0 cells (:2393): both are their own upwind node
+  const double gm = m * mu0 * omM;
+  const bool own_up = d ? first : last;
+  const bool edge = lane == (d ? 0 : 31);
+  const int from = own_up || edge ? lane : d ? lane - 1 : lane + 1;
+  const bool row_in = edge && !own_up;
+  const bool row_out = lane == (d ? 31 : 0) && warp_live;
+  const int up_in = first ? tid : tid - 1, up_out = last || tid == T - 1 ? tid : tid + 1;
+  __syncthreads();
+  if (active) b = (*mom(0, 0, tid) + *mom(0, 1, tid)) * omM;
+  __syncthreads();
+
+  for (int step = 0; step < nsteps; ++step) {
+    const int p = step & 1;
+    if (bc_node) {  // the seed boundary (:2361-2370)
+#pragma unroll
+      for (int j = 0; j < H; ++j) f[j] = bc[3 * i];
+      b = bc[3 * i + 1];
+      F = bc[3 * i + 2];
+    }
+    *mom(p, d, tid) = F;
+    if (row_out) {
+      const int w = d ? warp + 1 : warp - 1;
+      if (w >= 0 && w < W) {
+        double *dst = in(p, d, w);
+#pragma unroll
+        for (int j = 0; j < H; ++j) dst[j] = f[j];
+      }
+    }
+    // what stays of b, formed while the rows travel
+    b = fma(-gm, F, b);
+    __syncthreads();
+    if (warp_live) {
+      const double *up = in(p, d, warp);
+      b = fma(-gm, *mom(p, 1 - d, tid), b);
+      b = fma(gm, *mom(p, 1, up_in), fma(gm, *mom(p, 0, up_out), b));
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        if (j < HLO || j < nmax) {
+          double n = __shfl_sync(FULL, f[j], from);
+          if (row_in) n = up[j];
+          const double2 a = tab[j * T + tid];
+          f[j] = fma(a.x, f[j], fma(a.y, n, b));
+          F = j ? fma(rho[j], f[j], F) : f[0];
+        }
+      }
+    }
+  }
+
+  if (active) {
+    int code = 0, bad = 0, mu = 0;  // the first value that is not a number or infinite
+    const int k = r.list[sN + i];
+#pragma unroll
+    for (int j = 0; j < H; ++j)
+      if (j < nd) {
+        if (bad_value(f[j], &code) && !bad) bad = code, mu = at + sg * j;
+        f[j] = f[j] < DBL_MIN ? DBL_MIN : f[j];
+      }
+    if (bad) set_error(r, bad, 1, s, k, e, mu);
+    // node k and the thinned nodes that reference it (previous list node + 1 .. k)
+    const int kfirst = (i == 0) ? 0 : r.list[sN + i - 1] + 1;
+    for (int kk = kfirst; kk <= k; ++kk) {
+      double *op = reinterpret_cast<double *>(r.f) + ((sN + kk) * r.E + e) * M + at;
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        if (j < nd) *op = f[j];
+        op += sg;
+      }
+    }
+  }
+}
+
 // The CTA and cluster of a run: the fewest CTAs that hold a stream of N
 // nodes, of equal width in whole warps, so that no idle warp takes part in the
 // barriers.  Splitting a slab further does not pay (per launch, 24 x 400 x 20
@@ -287,7 +465,12 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
 // CTA's.  False where the mu grid does not mirror, a half of mu has more than 32
 // cells or a portable cluster (8 CTAs) cannot hold the stream; those runs keep
 // the kernel of stream.cu, which takes any mu grid and longer streams.
-bool stream64_shape(int N, int M, int m0, bool mirror_ok, StreamPlan *plan) {
+// The short streams' kernel, by the warps per SM that a launch of the other one
+// would have (12 energies, 10 sub-steps, ms of the other one and of this one): M
+// = 6, N = 64, 3.8 warps 0.56 and 0.44, 8.5 0.68 and 0.68, 15 0.86 and 0.95; M =
+// 20, N = 128, 1.9 2.88 and 2.44, 17 4.64 and 4.12, 30 6.5 and 6.6; M = 40, N =
+// 64, 3.8 2.83 and 1.78, 15 4.28 and 3.71; N = 96, 23 7.69 and 7.79.
+bool stream64_shape(int N, int M, int m0, bool mirror_ok, long long slabs, StreamPlan *plan) {
   if (!mirror_ok || m0 < 1 || (2 * m0 != M && 2 * m0 != M - 1 && 2 * m0 != M + 1)) return false;
   const int n = m0 > M - m0 ? m0 : M - m0;
   int h = 0, tmax = 0;
@@ -302,6 +485,9 @@ bool stream64_shape(int N, int M, int m0, bool mirror_ok, StreamPlan *plan) {
   plan->threads = ((N + cl - 1) / cl + 31) / 32 * 32;
   plan->cluster = (N + plan->threads - 1) / plan->threads;
   plan->reg_coef = 3;
+  // the short streams' kernel while a launch has few warps per SM
+  if (N <= kS64ShortNodes && slabs * (plan->threads / 32) <= 152 * (h < 10 ? 6 : 17))
+    plan->reg_coef = 4;
   plan->packed = plan->filled = plan->mirror = 0;
   plan->npt = 1;
   return true;
@@ -310,14 +496,15 @@ bool stream64_shape(int N, int M, int m0, bool mirror_ok, StreamPlan *plan) {
 template <int H, int HLO, int TMAX>
 static cudaError_t launch_stream64_t(const RunView &r, const StreamPlan &pl, int m0,
                                      cudaStream_t st) {
-  auto kern = k_stream64<H, HLO, TMAX>;
-  const size_t dyn = stream64_smem<H>(pl.threads);
+  const bool brief = pl.reg_coef == 4;
+  auto kern = brief ? k_stream64_short<H, HLO> : k_stream64<H, HLO, TMAX>;
+  const size_t dyn = brief ? stream64_short_smem<H>(pl.threads) : stream64_smem<H>(pl.threads);
   cudaError_t err =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
   if (err != cudaSuccess) return err;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(pl.cluster, r.S, r.E);
-  cfg.blockDim = dim3(pl.threads, 1, 1);
+  cfg.blockDim = dim3(brief ? 2 * pl.threads : pl.threads, 1, 1);
   cfg.dynamicSmemBytes = dyn;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];

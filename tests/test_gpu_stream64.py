@@ -58,6 +58,16 @@ def test_widest_block_of_a_bin(nodes, mu, oracle_lib):
     assert _check(_streaming(nodes, mu), oracle_lib).startswith("k_stream64")
 
 
+@pytest.mark.parametrize("rows,nodes,energies,mu,kernel", [
+    (4, 40, 8, 6, "k_stream64<6>"), (4, 33, 14, 21, "k_stream64<24>"),
+    (4, 64, 14, 40, "k_stream64<40>"), (1, 128, 3, 7, "k_stream64_short<8>"),
+    (1, 128, 3, 64, "k_stream64_short<64>"), (1, 129, 3, 7, "k_stream64<8>")])
+def test_short_streams_few_and_many(rows, nodes, energies, mu, kernel, oracle_lib):
+    w = W.custom(rows, rows, nodes, energies, mu, e_max=1.0, num_ep_steps=1,
+                 use_adiabatic_focus=0, use_adiabatic_change=0)
+    assert _check(w, oracle_lib).startswith(kernel)
+
+
 @pytest.mark.parametrize("m0", [0, 2, 7, 10])
 def test_mu_grid_that_does_not_mirror(m0, oracle_lib):
     w = _streaming(60, 10)
