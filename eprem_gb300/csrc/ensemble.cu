@@ -627,6 +627,15 @@ extern "C" int eprem_gpu_ensemble_step(eprem_gpu_ensemble *e) {
     const int rc = ensemble_capture(e);
     if (rc) return rc;
   }
+  // what the runs have queued on their own streams (uploads from page-locked
+  // memory, updates) comes first; inside a capture the caller orders it
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(e->origin, &cap));
+  for (eprem_gpu_run *r : e->runs)
+    if (cap == cudaStreamCaptureStatusNone) {
+      CK(cudaEventRecord(e->fork, r->stream));
+      CK(cudaStreamWaitEvent(e->origin, e->fork, 0));
+    }
   CK(cudaGraphLaunch(e->exec, e->origin));
   for (size_t i = 0; i < e->runs.size(); i++) e->runs[i]->launches += e->launches_per_step[i];
   return EPREM_GPU_OK;
