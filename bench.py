@@ -43,13 +43,14 @@ UNIT = "cell-updates/s"
 FLOPS_PER_CELL_SUBCYCLE = {"stream": 8.0, "focus": 11.0, "change": 11.0}
 BYTES_PER_CELL_UPDATE = {"fp64": 32.0, "fp32": 16.0}
 # DRAM bytes (read + write) per cell per launch of the dominant kernel, from
-# one ncu capture of the 96-stream subset (profiles/k_stream2_mirror_fp32_96streams.txt,
-# profiles/k_stream_fp64_96streams.txt, profiles/k_focus32_k_change32_fp32_96streams.txt):
+# one ncu capture of the 96-stream subset (profiles/k_stream2m_k_node32_fp32_96streams.txt,
+# profiles/k_stream64_k_node64_fp64_96streams.txt):
 # traffic per launch / 96*1000*50*40 cells; traffic grows with the number of
 # (stream, energy) slabs, so it scales to a full launch by the cells processed.
-NCU_DRAM_BYTES_PER_CELL = {("stream", "fp32"): 1603.9058e6 / 192e6,
-                           ("stream", "fp64"): 3054.831e6 / 192e6,
-                           ("node", "fp32"): 1488.048e6 / 192e6}
+NCU_DRAM_BYTES_PER_CELL = {("stream", "fp32"): 1599.6e6 / 192e6,
+                           ("stream", "fp64"): 3055.1e6 / 192e6,
+                           ("node", "fp32"): 1501.7e6 / 192e6,
+                           ("node", "fp64"): 3024.5e6 / 192e6}
 
 
 # ---------------------------------------------------------------------------
@@ -283,6 +284,8 @@ def roofline(kt, stats, steps, peak_tflops, hbm_peak, cells, form, stream_kernel
     kind = max(("stream", "node"), key=lambda k: kt[k][1])
     launches, total_ms = kt[kind]
     fl = flops_of(stats)[kind]
+    if kind == "stream" and (stream_kernel or "").startswith("k_stream64"):
+        fl *= 6.0 / FLOPS_PER_CELL_SUBCYCLE["stream"]  # three multiply-adds, not four
     per_launch_flops = fl / launches
     mean_s = total_ms / launches * 1e-3
     achieved = per_launch_flops / mean_s / 1e12
@@ -291,7 +294,7 @@ def roofline(kt, stats, steps, peak_tflops, hbm_peak, cells, form, stream_kernel
     return {
         "kernel": ((stream_kernel or {"fp32": "k_stream2", "fp64": "k_stream"}[form])
                    if kind == "stream"
-                   else {"fp32": "k_focus32+k_change32", "fp64": "k_node"}[form]),
+                   else {"fp32": "k_node32", "fp64": "k_node64"}[form]),
         "bound": "fp64" if form == "fp64" else "fp32",
         "achieved": round(achieved, 3), "peak": round(peak_tflops, 3), "unit": "TFLOP/s",
         "frac": round(achieved / peak_tflops, 4),

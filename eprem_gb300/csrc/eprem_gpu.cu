@@ -697,9 +697,9 @@ extern "C" int eprem_gpu_update_energetic_particles(eprem_gpu_run *r, double t_g
 // chunks; chunk c's host-to-device copy runs on the copy stream while chunk
 // c-1 is updated on the run's stream, and its device-to-host copy while chunk
 // c+1 is updated (measured on a GB300 whose host link moved 31 GB/s back:
-// 0.26-0.30 s of copies left per 4.81 s step with eight equal chunks).  The FP32 form converts each chunk in one of two staging
-// buffers (chunk c in buffer c % 2, reused once chunk c-2's copy back has
-// left it).  Synchronous: f_out holds the result on return.
+// 0.26-0.30 s of copies left per 4.81 s step with eight equal chunks).  The FP32
+// form converts each chunk in one of two staging buffers (chunk c in buffer
+// c % 2, reused once chunk c-2's copy back has left it).  Synchronous: f_out holds the result on return.
 extern "C" int eprem_gpu_update_energetic_particles_host(eprem_gpu_run *r, const double *f_in,
                                                          double *f_out, size_t stream_pitch,
                                                          double t_global) {

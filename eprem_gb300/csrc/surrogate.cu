@@ -9,7 +9,7 @@
 // Split form.  The reference relaxes f towards its mu-average inside every
 // streaming sub-cycle (src/energeticParticles.c:2406-2426).  In the split
 // form streaming runs without it, and the node phase applies, per (node, E)
-// row, the focusing sub-cycles (the Euler upwind of k_focus32) followed by
+// row, the focusing sub-cycles (the Euler upwind of node32.cuh) followed by
 // one exact relaxation over the whole sub-step, f = iso + (f - iso) e with
 // e = exp(-dt / tau).  Both pieces conserve sum_mu f.
 //
