@@ -289,10 +289,18 @@ int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool 
     const int kind = variant % 8, shape = variant / 8;
     if (variant < 0 || kind == 1 || kind == 2) return EPREM_GPU_ERR_ARG;
     const bool own = (M == 20 || M == 40) && 2 * m0 == M;
-    if (kind == 6 || kind == 7)
-      return own && plan_stream2m(N, M, m0, bc, shape, slabs, plan) ? 0 : EPREM_GPU_ERR_ARG;
+    // no longer streams than stream2.cu's: what holds a run does not depend on
+    // its boundary, and the stream list is formed in shared memory (8,300 nodes)
+    StreamPlan held{};
+    const bool holds = plan_stream2(N, M, m0, true, false, 0, &held) == 0;
+    if (kind == 6 || kind == 7) {
+      // M = 40: the second width named is two nodes per thread, the third three
+      const int width = M == 40 && (shape == 2 || shape == 3) ? 5 - shape : shape;
+      return own && holds && plan_stream2m(N, M, m0, bc, width, slabs, plan) ? 0
+                                                                             : EPREM_GPU_ERR_ARG;
+    }
     const int old = stream2_shape_count(M);
-    if (kind != 3 && (shape == 0 || shape > old) &&
+    if (kind != 3 && holds && (shape == 0 || shape > old) &&
         (kind != 5 || stream2_filled(M, m0)) &&
         plan_stream2m(N, M, m0, mirror_ok, shape ? shape - old : 0, slabs, plan))
       return 0;

@@ -112,3 +112,24 @@ def test_stream_plan_refusals(lib):
         runtime.plan_stream(100000, 40, 20, abi.EPREM_FP32, 0)
     fp64 = runtime.plan_stream(1000, 40, 20, abi.EPREM_FP64, 0)
     assert fp64["kind"] == 0 and fp64["slots"] >= 1000
+
+
+@pytest.mark.parametrize("mu,longest", [(2, 8192), (4, 8192), (9, 8192), (20, 8192), (33, 8192),
+                                        (40, 8192), (41, 6144), (48, 6144), (49, 4096),
+                                        (64, 4096)])
+@pytest.mark.parametrize("bc", [True, False])
+def test_longest_stream_of_a_mu_count(lib, mu, longest, bc):
+    """What an FP32 run may hold is fixed by its mu count, whichever kernel
+    streams it."""
+    for variant in (0, 4):
+        got = runtime.plan_stream(longest, mu, mu // 2, abi.EPREM_FP32, variant, bc)
+        assert got["slots"] >= longest and got["cluster"] <= 8
+        with pytest.raises(runtime.EpremGpuError):
+            runtime.plan_stream(longest + 1, mu, mu // 2, abi.EPREM_FP32, variant, bc)
+
+
+@pytest.mark.parametrize("shape,npt,longest", [(1, 4, 8189), (2, 2, 4093), (3, 3, 6142)])
+def test_named_widths_of_the_mirrored_kernel(lib, shape, npt, longest):
+    for kind in (6, 7):
+        got = runtime.plan_stream(longest, 40, 20, abi.EPREM_FP32, kind + 8 * shape)
+        assert got["npt"] == npt and got["cluster"] <= 8
