@@ -14,18 +14,34 @@
 // the sum after the sub-cycle follows from the node's and its neighbours'
 // first moments before it, and with b = (1 - em) S' / M known beforehand
 //   f_j' = A_j f_j + (C_j f_up,j + b),  C_j = em c_j,  A_j = em - C_j,
-// two fused multiply-adds, and one more for the new F.  For a node's particle
-// number to be kept over 1e5 sub-cycles A_j + C_j must be em exactly: C_j is
-// rounded to a multiple of em's last place, which makes the difference exact.
-// b itself is carried, not S (b' = b + (1 - em) / M m (F_up - F)), and F in units
-// of the largest |mu|, mu_0's, whose cell then enters without an operation; b is
-// formed afresh from the cells at every launch.
+// two fused multiply-adds, and one more for the new F.  b itself is carried, not
+// S (b' = b + (1 - em) / M m (F_up - F)), and F in units of the largest |mu|,
+// mu_0's, whose cell then enters without an operation.
+//
+// What that costs in precision is made good every kAnew sub-cycles:
+//   * b keeps an error of the last place of the largest value that it had, so it
+//     is formed anew from the cells: a node that drains by decades (weak
+//     scattering, a pulse that has passed) would otherwise end with it (5e-9 of f
+//     after 13,000 sub-cycles behind a pulse of 1e15).
+//   * for a node's particle number to be kept over 1e5 sub-cycles A_j + C_j must be
+//     em exactly, so C_j is a multiple of em's last place, which makes the
+//     difference exact.  Rounded once for all it would move f at a speed that is
+//     off by up to 1e-16 em / C_j; so it is rounded anew with a dither of up to
+//     half a place that steps by the golden ratio, from a start that f's own bits
+//     set, and its mean over any longer time is the coefficient itself.
+// Against long double over 1,344 model streams (2 to 40 mu cells, 100 to 13,000
+// sub-cycles, scattering from 1e-8 to 0.9 per sub-cycle, pulses of up to 1e15 and
+// segments of up to 1 : 1000) the largest error is 1.07 of the four-operation
+// form's in the geometric mean and its root mean square 0.76 (without the two:
+// 2.6e6 times it where a node drains); the worst of all is 1.6e-13, in the first
+// cells of a front of 1e15, against 8.3e-13.  It adds 8 operations per slot to the
+// 6 kAnew of that many sub-cycles.
 //
 // The mu grid's cells mirror each other, so cell j and cell M - 1 - j share one
-// {A, C}: 16 bytes of shared memory per slot and thread ([slot][thread], one
-// load).  A half without an upwind node (the first list node's mu >= 0 cells,
-// the last one's mu < 0 cells) takes its own cells as the upwind ones instead of
-// a C of its own.  Padding cells have C = |mu| = 0; what they hold goes nowhere.
+// {A, C}, from the mean of their |mu|: 16 bytes of shared memory per slot and
+// thread ([slot][thread], one load).  A half without an upwind node (the first
+// list node's mu >= 0 cells, the last one's mu < 0 cells) takes its own cells as
+// the upwind ones instead of a C of its own.  Padding cells have C = |mu| = 0; what they hold goes nowhere.
 //
 // Measured on a GB300, per launch, against the four-operation kernel of
 // stream.cu with its fixed CTA widths: 6 streams x 1000 x 50 x 40, 17.9 ->
@@ -56,27 +72,44 @@ namespace eprem {
   X(12, 10, 512) X(14, 12, 512) X(16, 14, 512) X(20, 16, 512) X(24, 20, 384) X(32, 24, 256)
 
 constexpr int kS64ShortNodes = 128;
+constexpr int kAnew = 32;  // sub-cycles between two sums and roundings (a power of two)
 
 template <int H>
 constexpr size_t stream64_short_smem(int nodes) {
   return sizeof(double2) * H * nodes +
-         sizeof(double) * (2 * 2 * (nodes / 32 * H + nodes) + H + 9);
+         sizeof(double) * (2 * 2 * (nodes / 32 * H + nodes) + 2 * nodes + 2 * H + 9);
 }
 
 template <int H>
 constexpr size_t stream64_smem(int threads) {
   return sizeof(double2) * H * threads + sizeof(double) * 2 * 2 * (threads / 32 + 1) * (H + 1) +
-         sizeof(double) * (H + 9);
+         sizeof(double) * (2 * H + 9);
 }
 
-// x (0 <= x < em) to the nearest multiple of em's last place, so that em - x
-// is exact: adding and taking off 1.5 * 2^52 of those places rounds it.
-__device__ __forceinline__ double to_place_of(double em, double x) {
-  const long long ex = __double_as_longlong(em) & 0x7ff0000000000000LL;
-  // em = 1: the last place of the values below it
-  const double p = __longlong_as_double(em >= 1.0 ? 0x3fe0000000000000LL : ex);
-  const double k = 1.5 * p;  // 1.5 * 2^52 * (p * 2^-52)
-  return __dsub_rn(__dadd_rn(x, k), k);
+// Rounds x (0 <= x < em) to a multiple of em's last place, so that em - x is
+// exact: adding and taking off 1.5 * 2^52 of those places does it.  dither: the
+// next step of `phase`, below half a place either way.
+struct PlaceOf {
+  double k, dither;
+  __device__ __forceinline__ PlaceOf(double em, uint32_t &phase) {
+    const long long ex = __double_as_longlong(em) & 0x7ff0000000000000LL;
+    // em = 1: the last place of the values below it
+    const double p = __longlong_as_double(em >= 1.0 ? 0x3fe0000000000000LL : ex);
+    k = 1.5 * p;  // 1.5 * 2^52 * (p * 2^-52)
+    dither = (double)(int)(phase | 1u) * (p * 0x1p-84);
+    phase += 2654435769u;  // 2^32 / golden ratio
+  }
+  __device__ __forceinline__ double operator()(double x) const {
+    return __dsub_rn(__dadd_rn(x, k), k);
+  }
+};
+// Where the dither of a node starts in a launch.
+__device__ __forceinline__ uint32_t dither_start(double f0, int i) {
+  return (uint32_t)__double2loint(f0) * 2654435769u + (uint32_t)i * 0x9e3779b1u;
+}
+// |mu| of slot j < m0: its two cells' mean.
+__device__ __forceinline__ double slot_mu(const RunView &r, int j) {
+  return 0.5 * (fabs(r.mugrid[j]) + fabs(r.mugrid[r.M - 1 - j]));
 }
 
 // the shared memory of CTA `rank` of the cluster at this CTA's `p`, and a store there
@@ -103,7 +136,8 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
   // warp w (mu >= 0); lo(p, w), the row of warp w's first thread (mu < 0)
   double *halo = reinterpret_cast<double *>(tab + H * T);
   double *rho = halo + 2 * 2 * (W + 1) * HP;  // [H] |mu| over its largest
-  double *bc = rho + H;  // [3][3] of the boundary's nodes: a cell, b, F
+  double *mus = rho + H;  // [H] |mu|
+  double *bc = mus + H;   // [3][3] of the boundary's nodes: a cell, b, F
   auto hi = [&](int p, int w) { return halo + ((p * 2 + 0) * (W + 1) + w) * HP; };
   auto lo = [&](int p, int w) { return halo + ((p * 2 + 1) * (W + 1) + w) * HP; };
 
@@ -133,8 +167,11 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
     atomicAdd(&r.status->stream_cs, (unsigned long long)nsteps * L * M);
   }
   for (int j = tid; j < 2 * 2 * (W + 1) * HP; j += T) halo[j] = 0.0;
-  const double mu0 = fabs(r.mugrid[0]);
-  for (int j = tid; j < H; j += T) rho[j] = j < nL ? fabs(r.mugrid[j]) / mu0 : 0.0;
+  const double mu0 = slot_mu(r, 0);
+  for (int j = tid; j < H; j += T) {
+    mus[j] = j < nL ? slot_mu(r, j) : 0.0;
+    rho[j] = mus[j] / mu0;
+  }
   __syncthreads();
 
   const int i = crank * T + tid;
@@ -158,29 +195,25 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
     row = reinterpret_cast<const double *>(r.f) + (g * r.E + e) * M;
     m = mult * (ec.vgrid * dtProp);
   }
-  double S = 0.0, sum = 0.0;  // sum: of rho
+  double sum = 0.0;  // of rho
 #pragma unroll
   for (int j = 0; j < H; ++j) {
     sum += rho[j];
     // few rows' loads in flight at a time: all of them together would spill
     if (j % 4 == 0) asm volatile("" ::: "memory");
     fL[j] = fR[j] = 0.0;
-    double c = 0.0;
     if (active && j < nL) {
       const double v = row[j];
       fL[j] = (r.check_seed && v < seedv) ? seedv : v;
-      c = to_place_of(em, em * (m * (rho[j] * mu0)));
     }
     if (active && j < nR) {
       const double v = row[M - 1 - j];
       fR[j] = (r.check_seed && v < seedv) ? seedv : v;
     }
-    tab[j * T + tid] = make_double2(active && j < nmax ? em - c : 0.0, c);
-    S += fL[j] + fR[j];
     FL = fma(rho[j], fL[j], FL);
     FR = fma(rho[j], fR[j], FR);
   }
-  b = S * omM;
+  uint32_t phase = dither_start(fL[0], i);
   if (bc_node) {
     bc[3 * i] = seedv;
     bc[3 * i + 1] = M * seedv * omM;
@@ -199,6 +232,19 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
 
   for (int step = 0; step < nsteps; ++step) {
     const int p = step & 1;
+    if (step % kAnew == 0) {
+      double S = 0.0;
+      const PlaceOf place(em, phase);
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        if (j < HLO || j < nmax) {
+          const double c = place(fma(em, m * mus[j], place.dither));
+          tab[j * T + tid] = make_double2(em - c, c);
+          S += (j < nL ? fL[j] : 0.0) + (j < nR ? fR[j] : 0.0);
+        }
+      }
+      b = S * omM;
+    }
     if (bc_node) {  // the seed boundary (:2361-2370)
 #pragma unroll
       for (int j = 0; j < H; ++j) fL[j] = fR[j] = bc[3 * i];
@@ -303,8 +349,10 @@ __global__ void __launch_bounds__(2 * kS64ShortNodes, 1) k_stream64_short(RunVie
   // the thread before it (mu >= 0)
   double *halo = reinterpret_cast<double *>(tab + H * T);
   double *Fs = halo + 2 * 2 * W * H;  // [2][2][T] F
-  double *rho = Fs + 2 * 2 * T;       // [H] |mu| over its largest
-  double *bc = rho + H;               // [3][3] of the boundary's nodes: a cell, b, F
+  double *Ss = Fs + 2 * 2 * T;        // [2][T] a direction's sum of cells
+  double *rho = Ss + 2 * T;           // [H] |mu| over its largest
+  double *mus = rho + H;              // [H] |mu|
+  double *bc = mus + H;               // [3][3] of the boundary's nodes: a cell, b, F
   auto in = [&](int p, int d, int w) { return halo + ((p * 2 + d) * W + w) * H; };
   auto mom = [&](int p, int d, int t) { return Fs + (p * 2 + d) * T + t; };
 
@@ -333,8 +381,11 @@ __global__ void __launch_bounds__(2 * kS64ShortNodes, 1) k_stream64_short(RunVie
     atomicAdd(&r.status->stream_cs, (unsigned long long)nsteps * L * M);
   }
   for (int j = threadIdx.x; j < 2 * 2 * (W * H + T); j += 2 * T) halo[j] = 0.0;
-  const double mu0 = fabs(r.mugrid[0]);
-  for (int j = threadIdx.x; j < H; j += 2 * T) rho[j] = j < nL ? fabs(r.mugrid[j]) / mu0 : 0.0;
+  const double mu0 = slot_mu(r, 0);
+  for (int j = threadIdx.x; j < H; j += 2 * T) {
+    mus[j] = j < nL ? slot_mu(r, j) : 0.0;
+    rho[j] = mus[j] / mu0;
+  }
   __syncthreads();
 
   const int i = tid;
@@ -359,7 +410,7 @@ __global__ void __launch_bounds__(2 * kS64ShortNodes, 1) k_stream64_short(RunVie
     row = reinterpret_cast<const double *>(r.f) + (g * r.E + e) * M + at;
     m = mult * (ec.vgrid * dtProp);
   }
-  double S = 0.0, sum = 0.0;  // sum: of rho
+  double sum = 0.0;  // of rho
 #pragma unroll
   for (int j = 0; j < H; ++j) {
     sum += rho[j];
@@ -370,14 +421,9 @@ __global__ void __launch_bounds__(2 * kS64ShortNodes, 1) k_stream64_short(RunVie
       const double v = row[sg * j];
       f[j] = (r.check_seed && v < seedv) ? seedv : v;
     }
-    if (!d) {
-      const double c = active && j < nL ? to_place_of(em, em * (m * (rho[j] * mu0))) : 0.0;
-      tab[j * T + tid] = make_double2(active && j < nmax ? em - c : 0.0, c);
-    }
-    S += f[j];
     F = fma(rho[j], f[j], F);
   }
-  if (active) *mom(0, d, tid) = S;
+  uint32_t phase = dither_start(f[0], i);
   if (bc_node && !d) {
     bc[3 * i] = seedv;
     bc[3 * i + 1] = M * seedv * omM;
@@ -393,11 +439,26 @@ __global__ void __launch_bounds__(2 * kS64ShortNodes, 1) k_stream64_short(RunVie
   const bool row_out = lane == (d ? 31 : 0) && warp_live;
   const int up_in = first ? tid : tid - 1, up_out = last || tid == T - 1 ? tid : tid + 1;
   __syncthreads();
-  if (active) b = (*mom(0, 0, tid) + *mom(0, 1, tid)) * omM;
-  __syncthreads();
 
   for (int step = 0; step < nsteps; ++step) {
     const int p = step & 1;
+    if (step % kAnew == 0) {
+      double S = 0.0;
+#pragma unroll
+      for (int j = 0; j < H; ++j)
+        if (j < HLO || j < nmax) S += j < nd ? f[j] : 0.0;
+      Ss[d * T + tid] = S;
+      __syncthreads();  // the last sub-cycle's table has been read, too
+      b = (Ss[tid] + Ss[T + tid]) * omM;
+      const PlaceOf place(em, phase);  // a direction's thread takes every second slot
+#pragma unroll
+      for (int j = 0; j < H; j += 2) {
+        if (j + d < HLO || j + d < nmax) {
+          const double c = place(fma(em, m * mus[j + d], place.dither));
+          tab[(j + d) * T + tid] = make_double2(em - c, c);
+        }
+      }
+    }
     if (bc_node) {  // the seed boundary (:2361-2370)
 #pragma unroll
       for (int j = 0; j < H; ++j) f[j] = bc[3 * i];
