@@ -333,18 +333,26 @@ __global__ void __launch_bounds__(kNode32MaxThreads)
       const int x0 = xs[it] + kRowTop;
       const float l2 = fminf(fmaxf(floorf(top), -1.0e6f), 1.0e6f);
       const int x1 = clamp_exp(x0 - (int)l2), up = x1 - x0 + kRowTop;
-      const float scale = up >= -126 ? pow2f(min(up, 127)) : 0.f;
-      // nothing near the floor or the far tail, up within float, no NaN or Inf
+      // nothing near the floor or the far tail, the shift within float, the
+      // exponential too, no NaN or Inf
       if (least > -115.f && least + (float)up > -125.f && up <= 127 && fabsf(sum) < 1e9f &&
-          top + (float)up < 127.f) {
+          top < 127.f) {
+        const float scale = pow2f(up);  // up >= kRowTop - 126
 #pragma unroll
         for (int m = 0; m < P; ++m) fr[m] = ex2(fr[m]) * scale;
       } else {
+        // a row that rose or fell by so many powers of two that 2^l or 2^up alone
+        // leaves float: its whole part joins the shift (which is kRowTop then,
+        // unless the exponent stopped at its limit)
+        const bool far = top >= 127.f || up > 127;
+        const float whole = far ? l2 : 0.f;
+        const int sh = far ? up + (int)l2 : up;
+        const float scale = sh > 127 ? INFINITY : sh >= -126 ? pow2f(sh) : 0.f;
         int code = 0;
 #pragma unroll
         for (int m = 0; m < P; ++m)
           if (m < LO || m < M) {
-            const float v = exp2_rel(fr[m], scale);
+            const float v = exp2_rel(fr[m] - whole, scale);
             if (bad_value(v, &code))
               set_error(r, code, 3, (int)((g0 + n) / N), (int)((g0 + n) % N), it - n * E, m);
             fr[m] = v < FLT_MIN ? FLT_MIN : v;
