@@ -75,6 +75,17 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// fmaxf and fminf that keep a NaN
+__device__ __forceinline__ float max_nan(float x, float y) {
+  float z;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(z) : "f"(x), "f"(y));
+  return z;
+}
+__device__ __forceinline__ float min_nan(float x, float y) {
+  float z;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(z) : "f"(x), "f"(y));
+  return z;
+}
 // log2 of a stored value less kRowTop.  The value is scaled by an exact power
 // of two first: by 2^-95 (the unit's error is absolute, 1e-7, where its argument
 // is near 1, as a row's leading cells then are), or more than 2^125 below the
@@ -221,8 +232,8 @@ __global__ void __launch_bounds__(kNode32MaxThreads)
         if (m < LO || m < M) {
           const float2 w = gm[m];
           const float q = fmaf(a, w.x, b * w.y);
-          qp[m] = fmaxf(q, 0.f);
-          qn[m] = fminf(q, 0.f);
+          qp[m] = max_nan(q, 0.f);  // a NaN face speed reaches f, as in the
+          qn[m] = min_nan(q, 0.f);  // reference's upwind flux
         }
       }
       for (int s = 0; s < c.ns_f; ++s) {
