@@ -34,7 +34,7 @@ __device__ __forceinline__ bool negative(double q) { return __double2hiint(q) < 
 __device__ __forceinline__ bool not_finite(double v) {
   return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
 }
-// v < DBL_MIN: negative or with a zero exponent
+// v < DBL_MIN of a finite v: negative or with a zero exponent
 __device__ __forceinline__ double floored(double v) {
   return __double2hiint(v) < 0x00100000 ? DBL_MIN : v;
 }
@@ -202,8 +202,10 @@ __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) 
       if (not_finite(v)) {
         const size_t g = g0 + n;
         set_error(r, nan_or_inf(v), 2, (int)(g / N), (int)(g % N), row - n * E, m);
+        v = v < DBL_MIN ? DBL_MIN : v;  // a NaN stays, whatever its sign bit
+      } else {
+        v = floored(v);
       }
-      v = floored(v);
     }
     if (change)
       f[row * pitch + m] = ln64(v, r.math64);
@@ -237,12 +239,15 @@ __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) 
   for (int i = tid; i < Gv * EM; i += T) {
     const int row = i / M, m = i - row * M, n = row / E;
     if (!nc[n].ok) continue;
-    const double v = exp64(f[row * pitch + m], r.math64);
+    double v = exp64(f[row * pitch + m], r.math64);
     if (not_finite(v)) {
       const size_t g = g0 + n;
       set_error(r, nan_or_inf(v), 3, (int)(g / N), (int)(g % N), row - n * E, m);
+      v = v < DBL_MIN ? DBL_MIN : v;
+    } else {
+      v = floored(v);
     }
-    fg[i] = floored(v);
+    fg[i] = v;
   }
 }
 
