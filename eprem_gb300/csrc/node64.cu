@@ -10,9 +10,10 @@
 //   * a face's scaled speed q is linear in the energy's a and in b with
 //     factors that depend on mu alone, one multiply-add; it is kept in shared
 //     memory over a row's sub-cycles;
-//   * a cell takes two multiply-adds, f - q f_up + q' f_up' , the upwind cell
-//     chosen by the sign bit of q (no FP64 compare), floors and NaN checks by
-//     the bits of the high word;
+//   * a cell takes three operations, f - (q f_up - q' f_up') with a flux carried
+//     to the next cell (third order: two multiply-adds), the upwind cell chosen by
+//     the sign bit of q (no FP64 compare), floors and NaN checks by the bits of the
+//     high word;
 //   * ln and exp (math64.cuh) run over the CTA's cells in order, every lane busy.
 // A CTA holds G whole nodes in shared memory; focusing takes a (node, energy)
 // row per thread, change a (node, mu) column, rows at an odd pitch (no bank
@@ -47,13 +48,38 @@ __device__ __forceinline__ int nan_or_inf(double v) {
 // cell at a time waits for shared memory each time.
 constexpr int kAhead = 4;
 
+// How a pass writes: the Euler operator alone, the Euler step that opens the third
+// order, or one of its mixed stages.  Alone, a cell is rounded once where it is
+// large: the difference of its faces' fluxes is formed first (three operations, a
+// flux carried from cell to cell; two multiply-adds on the cell itself round it
+// twice: the error of an FP64 step against 64 bits was 4.7e-16 at 24 x 400 x 20 x
+// 20 and 5.4e-16 at 6 x 1000 x 50 x 40 so, and is 4.2e-16 and 4.1e-16, for 1.5 and 5
+// ms of steps of 35 and 415).
+enum Pass { kEuler, kFirst, kMix };
+
 // One pass of the focusing operator over a row: the Euler step of `in`, g_m = in_m
 // - (q_{m+1} up_{m+1} - q_m up_m) with up the upwind cell and walls at both ends,
-// then out_m = c0 f_m + c1 g_m (EULER: g_m).  in and out may be the same row.
-template <bool EULER>
+// then out_m = c0 f_m + c1 g_m (kMix) or g_m.  in and out may be the same row.
+template <Pass PASS>
 __device__ __forceinline__ void focus_pass(const double *f, const double *in, double *out,
                                            const double *q, int M, double c0, double c1) {
+  // qp, up: the inner face and its upwind cell; kEuler: qp is its flux
   double cur = in[0], qp = 0.0, up = 0.0;
+  auto step = [&](double fm, double x, double w) {
+    const double un = negative(w) ? x : cur;
+    double g;
+    if (PASS == kEuler) {
+      const double flux = __dmul_rn(w, un);  // one value to both cells
+      g = cur - (flux - qp);
+      qp = flux;
+    } else {
+      g = fma(qp, up, fma(-w, un, cur));
+      qp = w;
+      up = un;
+    }
+    cur = x;
+    return PASS == kMix ? fma(c1, g, c0 * fm) : g;
+  };
   int m = 0;
   for (; m + kAhead < M; m += kAhead) {
     double x[kAhead], w[kAhead], o[kAhead];
@@ -61,48 +87,53 @@ __device__ __forceinline__ void focus_pass(const double *f, const double *in, do
     for (int j = 0; j < kAhead; ++j) {
       x[j] = in[m + 1 + j];
       w[j] = q[m + 1 + j];
-      o[j] = EULER ? 0.0 : f[m + j];
+      o[j] = PASS == kMix ? f[m + j] : 0.0;
     }
 #pragma unroll
-    for (int j = 0; j < kAhead; ++j) {
-      const double un = negative(w[j]) ? x[j] : cur;
-      const double g = fma(qp, up, fma(-w[j], un, cur));
-      o[j] = EULER ? g : fma(c1, g, c0 * o[j]);
-      cur = x[j];
-      qp = w[j];
-      up = un;
-    }
+    for (int j = 0; j < kAhead; ++j) o[j] = step(o[j], x[j], w[j]);
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) out[m + j] = o[j];
   }
   for (; m < M; ++m) {
     const bool wall = m + 1 == M;
     const double next = wall ? cur : in[m + 1], qn = wall ? 0.0 : q[m + 1];
-    const double un = negative(qn) ? next : cur;
-    const double g = fma(qp, up, fma(-qn, un, cur));
-    out[m] = EULER ? g : fma(c1, g, c0 * f[m]);
-    cur = next;
-    qp = qn;
-    up = un;
+    out[m] = step(PASS == kMix ? f[m] : 0.0, next, qn);
   }
 }
 
 // The same for the change operator on a column (stride `st`), with the seeds
 // b0, b1 flowing in at the ends; q_e = qa vw_{e-1} + qb at face e.
-template <bool EULER>
+template <Pass PASS>
 __device__ __forceinline__ void change_pass(const double *f, const double *in, double *out,
                                             const double *vw, int E, int st, double qa, double qb,
                                             double b0, double b1, double c0, double c1) {
-  auto mix = [&](double fe, double g) { return EULER ? g : fma(c1, g, c0 * fe); };
-  double cur = in[0], next = in[st];
+  auto mix = [&](double fe, double g) { return PASS == kMix ? fma(c1, g, c0 * fe) : g; };
+  double cur = in[0], next = in[st], prev = 0.0;
   double q = fma(qa, vw[0], qb);
-  double up = negative(q) ? next : cur;
+  double up = negative(q) ? next : cur;  // kEuler: the inner face's flux
   {  // first energy: downwind from above, or the seed below
     const double hi = negative(q) ? next : cur, lo = negative(q) ? cur : b0;
-    out[0] = mix(EULER ? 0.0 : f[0], fma(-q, hi - lo, cur));
+    out[0] = mix(PASS == kMix ? f[0] : 0.0, fma(-q, hi - lo, cur));
   }
-  double prev = cur;
+  if (PASS == kEuler) up = __dmul_rn(q, up);
+  prev = cur;
   cur = next;
+  auto step = [&](double fe, double x, double w) {
+    const double un = negative(w) ? x : cur;
+    double g;
+    if (PASS == kEuler) {
+      const double flux = __dmul_rn(w, un);  // one value to both cells
+      g = cur - (flux - up);
+      up = flux;
+    } else {
+      g = fma(q, up, fma(-w, un, cur));
+      up = un;
+    }
+    q = w;
+    prev = cur;
+    cur = x;
+    return mix(fe, g);
+  };
   int e = 1;
   for (; e + kAhead < E; e += kAhead) {
     double x[kAhead], w[kAhead], o[kAhead];
@@ -110,33 +141,20 @@ __device__ __forceinline__ void change_pass(const double *f, const double *in, d
     for (int j = 0; j < kAhead; ++j) {
       x[j] = in[(e + 1 + j) * st];
       w[j] = fma(qa, vw[e + j], qb);
-      o[j] = EULER ? 0.0 : f[(e + j) * st];
+      o[j] = PASS == kMix ? f[(e + j) * st] : 0.0;
     }
 #pragma unroll
-    for (int j = 0; j < kAhead; ++j) {
-      const double un = negative(w[j]) ? x[j] : cur;
-      o[j] = mix(o[j], fma(q, up, fma(-w[j], un, cur)));
-      prev = cur;
-      cur = x[j];
-      q = w[j];
-      up = un;
-    }
+    for (int j = 0; j < kAhead; ++j) o[j] = step(o[j], x[j], w[j]);
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) out[(e + j) * st] = o[j];
   }
   for (; e + 1 < E; ++e) {
-    next = in[(e + 1) * st];
-    const double qn = fma(qa, vw[e], qb);
-    const double un = negative(qn) ? next : cur;
-    out[e * st] = mix(EULER ? 0.0 : f[e * st], fma(q, up, fma(-qn, un, cur)));
-    prev = cur;
-    cur = next;
-    q = qn;
-    up = un;
+    const double x = in[(e + 1) * st], w = fma(qa, vw[e], qb);
+    out[e * st] = step(PASS == kMix ? f[e * st] : 0.0, x, w);
   }
   // last energy: upwind from below, or the seed above
   const double hi = negative(q) ? b1 : cur, lo = negative(q) ? cur : prev;
-  out[e * st] = mix(EULER ? 0.0 : f[e * st], fma(-q, hi - lo, cur));
+  out[e * st] = mix(PASS == kMix ? f[e * st] : 0.0, fma(-q, hi - lo, cur));
 }
 
 __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) {
@@ -180,13 +198,13 @@ __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) 
 #pragma unroll 4
       for (int m = 1; m < M; ++m) q[m] = fma(a, g1[m], gb[m]);
       if (r.focus_alg == 1) {
-        for (int s = 0; s < c.ns_f; ++s) focus_pass<true>(row, row, row, q, M, 0.0, 1.0);
+        for (int s = 0; s < c.ns_f; ++s) focus_pass<kEuler>(row, row, row, q, M, 0.0, 1.0);
       } else {
         double *st = wk2 + (size_t)it * pitch;
         for (int s = 0; s < c.ns_f; ++s) {
-          focus_pass<true>(row, row, st, q, M, 0.0, 1.0);
-          focus_pass<false>(row, st, st, q, M, 0.75, 0.25);
-          focus_pass<false>(row, st, row, q, M, 1.0 / 3.0, 2.0 / 3.0);
+          focus_pass<kFirst>(row, row, st, q, M, 0.0, 1.0);
+          focus_pass<kMix>(row, st, st, q, M, 0.75, 0.25);
+          focus_pass<kMix>(row, st, row, q, M, 1.0 / 3.0, 2.0 / 3.0);
         }
       }
     }
@@ -225,13 +243,13 @@ __global__ void __launch_bounds__(kNode64MaxThreads) k_node64(RunView r, int G) 
     const double qa = 0.5 * (c.step_c * c.cool) * am, qb = (c.step_c * c.cool) * bm;
     if (r.change_alg == 1) {
       for (int s = 0; s < c.ns_c; ++s)
-        change_pass<true>(col, col, col, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.0, 1.0);
+        change_pass<kEuler>(col, col, col, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.0, 1.0);
     } else {
       double *st = wk + (size_t)n * slab + m;
       for (int s = 0; s < c.ns_c; ++s) {
-        change_pass<true>(col, col, st, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.0, 1.0);
-        change_pass<false>(col, st, st, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.75, 0.25);
-        change_pass<false>(col, st, col, vw, E, pitch, qa, qb, c.bc0, c.bc1, 1.0 / 3.0, 2.0 / 3.0);
+        change_pass<kFirst>(col, col, st, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.0, 1.0);
+        change_pass<kMix>(col, st, st, vw, E, pitch, qa, qb, c.bc0, c.bc1, 0.75, 0.25);
+        change_pass<kMix>(col, st, col, vw, E, pitch, qa, qb, c.bc0, c.bc1, 1.0 / 3.0, 2.0 / 3.0);
       }
     }
   }
