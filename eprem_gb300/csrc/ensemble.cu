@@ -70,7 +70,7 @@ int tune_stream(eprem_gpu_run *r, int *chosen) {
     if (e != cudaSuccess) break;
     StreamPlan pl{};
     if (plan_stream(EPREM_FP32, r->dims.num_nodes, r->dims.num_mu, r->m0, variant,
-                    r->v.use_bc != 0, r->mirror_ok, r->slabs(), &pl))
+                    r->mirror_ok, r->slabs(), &pl))
       continue;
     if (launch_stream(v, pl, r->m0, r->stream, &dummy)) {  // warm-up
       e = cudaGetLastError();
@@ -119,7 +119,7 @@ extern "C" int eprem_gpu_plan_stream(int num_nodes, int num_mu, int m0, int prec
     return fail(EPREM_GPU_ERR_ARG, "bad sizes");
   StreamPlan p{};
   // (a run with few slabs may take a narrower shape)
-  if (plan_stream(precision, num_nodes, num_mu, m0, variant, seed_boundary != 0,
+  if (plan_stream(precision, num_nodes, num_mu, m0, variant,
                   precision == EPREM_FP64 || seed_boundary != 0, 1 << 20, &p))
     return fail(EPREM_GPU_ERR_ARG, "no streaming kernel fits these sizes");
   const bool s2 = p.reg_coef == 2;
@@ -154,7 +154,7 @@ extern "C" int eprem_gpu_set_stream_variant(eprem_gpu_run *r, int variant) {
   if (!r) return fail(EPREM_GPU_ERR_ARG, "null run");
   StreamPlan pl{};
   if (plan_stream(r->dims.precision, r->dims.num_nodes, r->dims.num_mu, r->m0, variant,
-                  r->v.use_bc != 0, r->mirror_ok, r->slabs(), &pl))
+                  r->mirror_ok, r->slabs(), &pl))
     return fail(EPREM_GPU_ERR_ARG, "streaming variant does not fit this run's sizes");
   r->splan = pl;
   r->params.stream_variant = variant;
@@ -276,7 +276,7 @@ extern "C" int eprem_gpu_ensemble_autotune(eprem_gpu_ensemble *e, int *chosen_va
     eprem_gpu_run *r = e->runs[i];
     StreamPlan key{};
     plan_stream(r->dims.precision, r->dims.num_nodes, r->dims.num_mu, r->m0, 0,
-                r->v.use_bc != 0, r->mirror_ok, r->slabs(), &key);
+                r->mirror_ok, r->slabs(), &key);
     const std::vector<int> k = {r->dims.precision, key.mmax, key.cluster, key.threads,
                                 r->dims.num_mu, r->m0};
     int variant = -1;

@@ -160,8 +160,8 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
     mirror64 = mirror64 && fabs(grids->mugrid[m] + grids->mugrid[M - 1 - m]) <= 4 * DBL_EPSILON &&
                fabs(grids->mugrid[m]) <= (1.0 + 4 * DBL_EPSILON) * fabs(grids->mugrid[0]);
   r->mirror_ok = dims->precision == EPREM_FP64 ? mirror64 : bc && even_mu;
-  int prc = plan_stream(dims->precision, N, M, m0, params->stream_variant, bc, r->mirror_ok,
-                        (long long)S * E, &r->splan);
+  int prc = plan_stream(dims->precision, N, M, m0, params->stream_variant,
+                        r->mirror_ok, (long long)S * E, &r->splan);
   const bool fast64 = dims->precision == EPREM_FP64 && params->adiabatic_focus_alg <= 2 &&
                       params->adiabatic_change_alg <= 2;
   if (!prc)

@@ -33,9 +33,10 @@ struct StreamPlan {
   int npt;       // stream2.cu: list nodes per thread
   int mirror;    // stream2m.cu (mmax is M itself there)
 };
-// bc: the run has the seed boundary (FP32's mirrored kernel needs it); mirror_ok:
-// FP32 form, and a uniform symmetric mu grid, FP64 form, a symmetric mu grid; slabs: (stream, energy) slabs of a launch
-int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool mirror_ok,
+// mirror_ok (eprem_gpu_run::mirror_ok): the mirrored kernels may run: FP32 form, the
+// seed boundary and a uniform symmetric mu grid, FP64 form, a symmetric mu grid;
+// slabs: (stream, energy) slabs of a launch
+int plan_stream(int precision, int N, int M, int m0, int variant, bool mirror_ok,
                 long long slabs, StreamPlan *plan);
 int launch_stream(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t st,
                   uint64_t *launches);

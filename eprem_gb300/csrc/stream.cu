@@ -270,7 +270,7 @@ static int threads_for(int mmax) {
 // (an odd mu half padded with a zero cell), 5 as 4 with the cell guards
 // resolved at compile time (M fills its bin, m0 = M/2), 6 and 7 the mirrored
 // kernel of stream2m.cu (the mu < 0 half in mirror order, one upwind
-// coefficient per two cells; M = 20 or 40, and the seed boundary).  Shape 0
+// coefficient per two cells; M = 20 or 40, and mirror_ok).  Shape 0
 // lets the planner choose from the sizes, k >= 1 names the k-th shape: of the
 // mu bin for 3 to 5, of the widths of M for 6 and 7.  The mirrored kernel
 // serves kinds 0, 4 and 5 with shape 0 too wherever it fits (mirror_ok: seed
@@ -283,7 +283,7 @@ static int threads_for(int mmax) {
 // The FP64 form has one kernel per stream length and mu grid (stream64.cu, or
 // k_stream where a cluster of that one cannot hold the stream, or the cells of
 // the mu grid do not mirror each other); variants 1 and 2 name it there.
-int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool mirror_ok,
+int plan_stream(int precision, int N, int M, int m0, int variant, bool mirror_ok,
                 long long slabs, StreamPlan *plan) {
   if (precision == EPREM_FP32) {
     const int kind = variant % 8, shape = variant / 8;
@@ -296,8 +296,9 @@ int plan_stream(int precision, int N, int M, int m0, int variant, bool bc, bool 
     if (kind == 6 || kind == 7) {
       // M = 40: the second width named is two nodes per thread, the third three
       const int width = M == 40 && (shape == 2 || shape == 3) ? 5 - shape : shape;
-      return own && holds && plan_stream2m(N, M, m0, bc, width, slabs, plan) ? 0
-                                                                             : EPREM_GPU_ERR_ARG;
+      return own && holds && plan_stream2m(N, M, m0, mirror_ok, width, slabs, plan)
+                 ? 0
+                 : EPREM_GPU_ERR_ARG;
     }
     const int old = stream2_shape_count(M);
     if (kind != 3 && holds && (shape == 0 || shape > old) &&

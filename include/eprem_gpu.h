@@ -136,7 +136,8 @@ typedef struct {
                                        mirrored kernel at M = 20 or 40: the
                                        mu < 0 half in mirror order, one upwind
                                        coefficient per two cells (needs the
-                                       seed boundary).  shape 0 automatic --
+                                       seed boundary and a uniform symmetric
+                                       mu grid).  shape 0 automatic --
                                        with kinds 0, 4 and 5 that is the
                                        mirrored kernel too, at any M from 4 to
                                        64, where the mu grid is uniform and
