@@ -270,15 +270,18 @@ extern "C" int eprem_gpu_ensemble_get_time(eprem_gpu_ensemble *e, double *t_glob
 
 extern "C" int eprem_gpu_ensemble_autotune(eprem_gpu_ensemble *e, int *chosen_variants) {
   if (!e) return fail(EPREM_GPU_ERR_ARG, "null ensemble");
-  // size class: precision, mu bin and cluster shape of the default plan
+  // size class: precision, mu count and default plan, and what decides which
+  // variants a run may take
   std::vector<std::pair<std::vector<int>, int>> classes;  // key -> variant
   for (size_t i = 0; i < e->runs.size(); i++) {
     eprem_gpu_run *r = e->runs[i];
     StreamPlan key{};
     plan_stream(r->dims.precision, r->dims.num_nodes, r->dims.num_mu, r->m0, 0,
                 r->mirror_ok, r->slabs(), &key);
-    const std::vector<int> k = {r->dims.precision, key.mmax, key.cluster, key.threads,
-                                r->dims.num_mu, r->m0};
+    const std::vector<int> k = {r->dims.precision, key.mmax,      key.cluster,
+                                key.threads,       key.npt,       key.mirror,
+                                r->dims.num_mu,    r->m0,         r->v.use_bc,
+                                r->v.use_stream,   r->mirror_ok};
     int variant = -1;
     for (auto &c : classes)
       if (c.first == k) variant = c.second;

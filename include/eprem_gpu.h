@@ -548,7 +548,8 @@ int eprem_gpu_ensemble_create(eprem_gpu_run *const *runs, int num_runs,
 int eprem_gpu_ensemble_destroy(eprem_gpu_ensemble *ens);
 int eprem_gpu_ensemble_set_time(eprem_gpu_ensemble *ens, const double *t_global);
 int eprem_gpu_ensemble_get_time(eprem_gpu_ensemble *ens, double *t_global);
-/* Autotune one run per size class (precision, mu bin, cluster shape) and give
+/* Autotune one run per size class (precision, mu count, default streaming plan,
+ * seed boundary, symmetry of the mu grid) and give
  * its choice to the others of the class; chosen_variants (may be NULL)
  * receives one variant per run.  The next step captures a new graph. */
 int eprem_gpu_ensemble_autotune(eprem_gpu_ensemble *ens, int *chosen_variants);
