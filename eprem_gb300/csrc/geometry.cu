@@ -227,10 +227,7 @@ int launch_geometry(const RunView &r, cudaStream_t st, double norm_radius, doubl
   else
     k_node_prep<false><<<blocks, t, 0, st>>>(r, norm_radius, neg_beta, mfp_type, mfp_power, bs_au);
   size_t smem = (size_t)r.N * (3 * sizeof(double) + sizeof(int));
-  // per launch: runs of different sizes share the kernel's attribute
-  if (cudaFuncSetAttribute(k_stream_list, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return EPREM_GPU_ERR_CUDA;
+  if (allow_smem((const void *)k_stream_list) != cudaSuccess) return EPREM_GPU_ERR_CUDA;
   k_stream_list<<<r.S, kListThreads, smem, st>>>(r);
   *launches += 2;
   return cudaGetLastError() == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
@@ -239,11 +236,8 @@ int launch_geometry(const RunView &r, cudaStream_t st, double norm_radius, doubl
 int geometry_smem_bytes(int N) { return N * (3 * (int)sizeof(double) + (int)sizeof(int)); }
 
 int setup_geometry_attrs(int N) {
-  int smem = geometry_smem_bytes(N);
-  if (cudaFuncSetAttribute(k_stream_list, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-      cudaSuccess)
-    return EPREM_GPU_ERR_CUDA;
-  return 0;
+  if (geometry_smem_bytes(N) > kSmemMost) return EPREM_GPU_ERR_CUDA;
+  return allow_smem((const void *)k_stream_list) == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }
 
 }  // namespace eprem

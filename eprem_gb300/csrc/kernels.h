@@ -13,6 +13,15 @@ namespace eprem {
 // (k_update_mhd, 1440 nodes: 50 us in CTAs of 256 threads, 28 of 32).
 inline int node_threads(size_t nodes) { return nodes <= (size_t)152 * 32 * 8 ? 32 : 128; }
 
+// The dynamic shared memory that a kernel whose launches differ in it is allowed:
+// the most that any of them may ask for, one value for all of them, since threads
+// with runs of other sizes set and launch the same kernels (a lower value set in
+// between would refuse a launch).  An SM's 227 KB less what kernels hold statically.
+constexpr int kSmemMost = 227 * 1024 - 2048;
+inline cudaError_t allow_smem(const void *kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
+}
+
 // geometry.cu
 // node_rates: also the node coefficients and sub-cycle counts (added to the
 // statistics) of the FP64 form's node64.cu, once per updateEnergeticParticles

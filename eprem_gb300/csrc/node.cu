@@ -503,8 +503,7 @@ int plan_node(int precision, int E, int M, NodePlan *plan) {
 template <typename Real, int P>
 static cudaError_t launch_node_t(const RunView &r, const NodePlan &pl, cudaStream_t st) {
   auto kern = k_node<Real, P>;
-  cudaError_t err =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+  cudaError_t err = allow_smem((const void *)kern);
   if (err != cudaSuccess) return err;
   const size_t SN = (size_t)r.S * r.N;
   const unsigned blocks = (unsigned)((SN + pl.nodes - 1) / pl.nodes);

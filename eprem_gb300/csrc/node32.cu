@@ -123,8 +123,7 @@ static cudaError_t launch_k(const NodePlan &pl, const RunView &r, int blocks,
   const void *kern = node32_kernel_a(pl.pmax, width(r.M));
   if (!kern) kern = node32_kernel_b(pl.pmax, width(r.M));
   if (!kern) return cudaErrorInvalidValue;
-  const cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+  const cudaError_t e = allow_smem(kern);
   if (e != cudaSuccess) return e;
   RunView v = r;
   int G = pl.nodes;

@@ -298,9 +298,7 @@ int plan_node64(int E, int M, int focus_alg, NodePlan *plan) {
 }
 
 int launch_node64(const RunView &r, const NodePlan &pl, cudaStream_t st, uint64_t *launches) {
-  if (cudaFuncSetAttribute(k_node64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) !=
-      cudaSuccess)
-    return EPREM_GPU_ERR_CUDA;
+  if (allow_smem((const void *)k_node64) != cudaSuccess) return EPREM_GPU_ERR_CUDA;
   const size_t SN = (size_t)r.S * r.N;
   const unsigned blocks = (unsigned)((SN + pl.nodes - 1) / pl.nodes);
   k_node64<<<blocks, pl.threads, pl.smem, st>>>(r, pl.nodes);

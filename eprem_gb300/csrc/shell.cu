@@ -557,8 +557,7 @@ __global__ void __launch_bounds__(kPerpThreads, 6) k_perp_slice(RunView r, PerpO
 template <typename Real, int V>
 static cudaError_t launch_perp_as(const RunView &r, const PerpOps &ops, cudaStream_t st) {
   const size_t smem = perp_smem<Real>(r.S, r.M, ops.L[0], ops.L[1]);
-  const cudaError_t e = cudaFuncSetAttribute(
-      k_perp_slice<Real, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem((const void *)k_perp_slice<Real, V>);
   if (e != cudaSuccess) return e;
   // as many blocks as run at once: six by their registers, fewer by shared memory
   const int fit = std::max(1, std::min(6, (int)(227 * 1024 / (smem + 1024))));

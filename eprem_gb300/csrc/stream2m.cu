@@ -129,9 +129,7 @@ int launch_stream2m(const RunView &r, const Stream2mView *views, const int4 *ite
 #undef EPREM_S2M_FIND
   if (!kern) return EPREM_GPU_ERR_ARG;
   const size_t dyn = smem_of(P, extra, pl.npt, pl.threads);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) !=
-      cudaSuccess)
-    return EPREM_GPU_ERR_CUDA;
+  if (allow_smem(kern) != cudaSuccess) return EPREM_GPU_ERR_CUDA;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = items ? dim3(pl.cluster * n_items, 1, 1) : dim3(pl.cluster, r.S, r.E);
   cfg.blockDim = dim3(pl.threads, 1, 1);

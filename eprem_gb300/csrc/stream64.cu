@@ -560,8 +560,7 @@ static cudaError_t launch_stream64_t(const RunView &r, const StreamPlan &pl, int
   const bool brief = pl.reg_coef == 4;
   auto kern = brief ? k_stream64_short<H, HLO> : k_stream64<H, HLO, TMAX>;
   const size_t dyn = brief ? stream64_short_smem<H>(pl.threads) : stream64_smem<H>(pl.threads);
-  cudaError_t err =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  cudaError_t err = allow_smem((const void *)kern);
   if (err != cudaSuccess) return err;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(pl.cluster, r.S, r.E);
