@@ -699,7 +699,8 @@ extern "C" int eprem_gpu_update_energetic_particles(eprem_gpu_run *r, double t_g
 // c+1 is updated (measured on a GB300 whose host link moved 31 GB/s back:
 // 0.26-0.30 s of copies left per 4.81 s step with eight equal chunks).  The FP32
 // form converts each chunk in one of two staging buffers (chunk c in buffer
-// c % 2, reused once chunk c-2's copy back has left it).  Synchronous: f_out holds the result on return.
+// c % 2, reused once chunk c-2's copy back has left it).  Synchronous: f_out
+// holds the result on return.
 extern "C" int eprem_gpu_update_energetic_particles_host(eprem_gpu_run *r, const double *f_in,
                                                          double *f_out, size_t stream_pitch,
                                                          double t_global) {
@@ -709,32 +710,33 @@ extern "C" int eprem_gpu_update_energetic_particles_host(eprem_gpu_run *r, const
   const size_t per_stream = (size_t)r->dims.num_nodes * r->dims.num_energies * r->dims.num_mu;
   const size_t pitch = stream_pitch ? stream_pitch : per_stream;
   if (pitch < per_stream) return fail(EPREM_GPU_ERR_ARG, "stream_pitch below N*E*M");
-  if (r->node_mode != EPREM_NODE_PHASE_REFERENCE || r->shell_on || r->drift_on) {
-    // those phases, shell diffusion and drift work on the whole run
+  // Chunks: a short first and last one (1/32 of the streams each: the first
+  // upload and the last download are the copies nothing hides) around up to
+  // six long ones, whose copies each take less than a neighbour's update.  The
+  // long ones hold kChunkSlabs (stream, energy) slabs or more on average (they
+  // are whole streams); a run that leaves fewer than two such goes in one piece,
+  // by the calls that upload, update and download: a launch over few slabs leaves
+  // SMs idle while its longest ones finish, which costs more than the copies, also
+  // where a step is one sub-step (ms of a step in eight chunks and in one: 54
+  // streams x 632 x 38 x 22, 2,052 slabs, FP32, 30 sub-steps 85 and 37, one 74 and
+  // 27; 90 x 1500 x 20 x 40, 1,800 slabs, 149 and 133, 121 and 100; 96 x 1600 x 25
+  // x 40, 2,400 slabs, 241 and 229, 187 and 178).
+  constexpr long long kChunkSlabs = 152 * 8;
+  const int edge = S >= 64 ? (S + 31) / 32 : (S >= 8 ? 1 : 0), mid = S - 2 * edge;
+  const int pieces =
+      (int)std::min<long long>(6, (long long)mid * r->dims.num_energies / kChunkSlabs);
+  if (!edge || pieces < 2 || r->node_mode != EPREM_NODE_PHASE_REFERENCE || r->shell_on ||
+      r->drift_on) {
+    // (other node phases, shell diffusion and drift work on the whole run)
     int rc = eprem_gpu_upload_f_pitched(r, f_in, pitch);
     if (!rc) rc = ep_update(r, r->v);
     if (!rc) rc = eprem_gpu_download_f_pitched(r, f_out, pitch);
     return rc;
   }
-  // Chunks: a short first and last one (1/32 of the streams each: the first
-  // upload and the last download are the copies nothing hides) around up to
-  // six long ones, whose copies each take less than a neighbour's update.  A
-  // chunk keeps at least kChunkSlabs (stream, energy) slabs, a run with fewer
-  // than twice that goes in one piece: a launch over few slabs leaves SMs idle
-  // while its longest ones finish, which costs more than the copies (54 streams
-  // x 632 x 38 x 22, 2052 slabs, a step of 30 sub-steps: 79 ms of streaming in
-  // eight chunks, 30 in one, and 5 ms of copies).
-  constexpr long long kChunkSlabs = 152 * 8;
-  std::vector<int> bounds{0};
-  const int pieces = (int)std::min<long long>(6, r->slabs() / kChunkSlabs);
-  const int edge = pieces < 2 ? 0 : S >= 64 ? (S + 31) / 32 : (S >= 8 ? 1 : 0);
-  if (edge) {
-    const int mid = S - 2 * edge;
-    bounds.push_back(edge);
-    for (int i = 1; i <= pieces; i++) {
-      const int b = edge + (int)((long long)mid * i / pieces);
-      if (b > bounds.back()) bounds.push_back(b);
-    }
+  std::vector<int> bounds{0, edge};
+  for (int i = 1; i <= pieces; i++) {
+    const int b = edge + (int)((long long)mid * i / pieces);
+    if (b > bounds.back()) bounds.push_back(b);
   }
   if (bounds.back() < S) bounds.push_back(S);
   const int nch = (int)bounds.size() - 1;

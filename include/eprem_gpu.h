@@ -282,9 +282,10 @@ int eprem_gpu_update_energetic_particles(eprem_gpu_run *run, double t_global);
  * caller holding f there packs nothing on the host.  (The drop-in keeps f on
  * the device across steps instead: eprem_gpu_ripple_f.)  f_in and f_out may
  * be the same array.  The streams go through in chunks (a short first and last
- * one around up to six long ones of at least 1216 (stream, energy) slabs; a run
- * of fewer than twice that goes in one), and each chunk's host-to-device copy,
- * update and device-to-host copy overlap the neighbouring chunks' work, so the
+ * one around up to six long ones of 1216 (stream, energy) slabs or more on
+ * average; a run that leaves fewer than two such goes in one piece), and each
+ * chunk's host-to-device copy, update and device-to-host copy overlap the
+ * neighbouring chunks' work, so the
  * copies hide behind the update when the host memory is page-locked
  * (eprem_gpu_host_alloc, or eprem_gpu_host_register on an existing
  * allocation).  Node fields are not copied: upload and download them as for
