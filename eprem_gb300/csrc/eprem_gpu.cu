@@ -649,6 +649,8 @@ int eprem::ep_node_phase(eprem_gpu_run *r, const RunView &v) {
     });
     return rc ? cuda_fail(cudaGetLastError(), "shell diffusion / drift launch") : EPREM_GPU_OK;
   }
+  if ((shell || drift) && !r->d_shell_f)
+    return fail(EPREM_GPU_ERR_STATE, "no second f buffer for shell diffusion or drift");
   // (each perpendicular step swaps the run's two f buffers, which v, the
   // run's own view, sees)
   // DiffuseShellData after every stream's sub-step (src/energeticParticles.c:178-182)
@@ -1034,9 +1036,10 @@ extern "C" int eprem_gpu_set_time_step(eprem_gpu_run *r, double t_del) {
 }
 
 // The second f buffer (and its row exponents) that a perpendicular step
-// writes before it becomes the run's f.
-static int ensure_second_f(eprem_gpu_run *r) {
-  if (r->d_shell_f) return EPREM_GPU_OK;
+// writes before it becomes the run's f, where the run's slices, with lists of
+// these lengths, are too large to be stepped in place.
+static int ensure_second_f(eprem_gpu_run *r, int shell_L, int drift_L) {
+  if (r->d_shell_f || perp_slice_fits(r->v, shell_L, drift_L)) return EPREM_GPU_OK;
   const size_t elem = r->dims.precision == EPREM_FP32 ? sizeof(float) : sizeof(double);
   CK(cudaMalloc(&r->d_shell_f, elem * r->cells() + 16));  // as d_f, tail zeroed as there
   CK(cudaMemset(r->d_shell_f, 0, elem * r->cells() + 16));
@@ -1113,8 +1116,11 @@ extern "C" int eprem_gpu_set_drift(eprem_gpu_run *r, const int32_t *news,
       const size_t elem = r->dims.precision == EPREM_FP32 ? sizeof(float) : sizeof(double);
       CK(cudaMalloc(&r->d_drift_del, elem * 4 * r->sn() * E));
     }
-    const int rc = ensure_second_f(r);
-    if (rc) return rc;
+    const int rc = ensure_second_f(r, r->shell_on ? r->shell_L : 0, L);
+    if (rc) {
+      r->drift_on = false;
+      return rc;
+    }
     cudaFree(r->d_drift_ent);
     r->d_drift_ent = nullptr;
     CK(cudaMalloc(&r->d_drift_ent, sizeof(int) * ent.size()));
@@ -1122,6 +1128,12 @@ extern "C" int eprem_gpu_set_drift(eprem_gpu_run *r, const int32_t *news,
     CK(cudaMemcpy(r->d_drift_ent, ent.data(), sizeof(int) * ent.size(), cudaMemcpyHostToDevice));
     r->drift_L = L;
     r->drift_links = true;
+  } else if (r->drift_links) {
+    const int rc = ensure_second_f(r, r->shell_on ? r->shell_L : 0, r->drift_L);
+    if (rc) {
+      r->drift_on = false;
+      return rc;
+    }
   }
   return EPREM_GPU_OK;
 }
@@ -1150,7 +1162,7 @@ extern "C" int eprem_gpu_set_shell_diffusion(eprem_gpu_run *r, const int32_t *ne
     CK(cudaMalloc(&r->d_news, sizeof(int) * 4 * (size_t)S));
     CK(cudaMalloc(&r->d_shell_del, sizeof(double) * 5 * r->sn() * r->dims.num_energies));
   }
-  rc = ensure_second_f(r);
+  rc = ensure_second_f(r, L, r->drift_on && r->drift_links ? r->drift_L : 0);
   if (rc) return rc;
   cudaFree(r->d_shell_ent);
   r->d_shell_ent = nullptr;

@@ -61,8 +61,9 @@ struct eprem_gpu_run {
   double *d_flux = nullptr;
   double *d_tmpl = nullptr;   // [S][E][M] template rows of eprem_gpu_ripple_f
   // shell diffusion (eprem_gpu_set_shell_diffusion): NEWS links, per-target
-  // gather lists (S x shell_L, padded with -1), per-call fractions and a
-  // second f buffer that each diffusion step writes and then swaps with d_f
+  // gather lists (S x shell_L, padded with -1), per-call fractions and, where
+  // slices do not fit shared memory, a second f buffer that each diffusion step
+  // writes and then swaps with d_f
   bool shell_on = false;
   double kperxkpar = 0.0;
   int shell_L = 0;

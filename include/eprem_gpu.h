@@ -341,8 +341,9 @@ int eprem_gpu_set_time_step(eprem_gpu_run *run, double t_del);
  * (face*R*C + row*C + col) of each stream's north, east, west and south
  * neighbour on its shell -- the Node_t links n, e, w, s of
  * src/cubeShellStruct.h that initNEWS / initCopyAll set, the same on every
- * shell; NULL switches the diffusion off.  Allocates the gather lists and an
- * f-sized scratch on the first call.  The diffusion couples the streams, so
+ * shell; NULL switches the diffusion off.  Allocates the gather lists and
+ * fractions on the first call, and an f-sized scratch where all streams' rows of
+ * one node and energy do not fit shared memory.  The diffusion couples the streams, so
  * eprem_gpu_update_energetic_particles_host then moves all of f in one copy
  * each way instead of pipelining chunks, and ensembles refuse such runs.
  * EPREM_GPU_ERR_ARG for a neighbour out of range or kperxkpar < 1e-33. */
