@@ -71,7 +71,13 @@ bool plan_stream2m(int N, int M, int m0, bool mirror_ok, int width, long long sl
     if (w.P != P) continue;
     ++k;
     if (width && k != width) continue;
-    const int need = (N + w.npt - 1 + w.npt - 1) / w.npt;  // threads
+    // threads: a list of L nodes ends at slot L + sh, a multiple of npt
+    // (stream2m.cuh), so a stream may fill its CTA.  The shapes that have numbers of
+    // their own (kinds 6 and 7, M = 20 and 40) keep the npt - 1 spare slots and the
+    // longest streams that they are known by.  (ms of four sub-steps, 96 streams x
+    // 16 E, one CTA and the cluster of three that a spare slot asked for: M = 64, N =
+    // 512 18.9 and 32.7; M = 48, N = 768 25.4 and 43.7; M = 36, N = 1024 30.0 and 52.8)
+    const int need = (N + w.npt - 1 + (M == 20 || M == 40 ? w.npt - 1 : 0)) / w.npt;
     int cl = 1, t = (need + 31) / 32 * 32;
     if (t > 256) {  // clusters of 128 threads, two CTAs to an SM, else of 256
       t = 128;
