@@ -35,8 +35,8 @@ struct StreamPlan {
   int mmax;      // register slots per thread (>= M)
   int threads;   // threads per CTA
   int cluster;   // CTAs per (stream, energy) slab
-  int reg_coef;  // coefficients in registers (1), shared memory (0); 2: stream2.cu;
-                 // 3: stream64.cu, 4: its kernel for short streams
+  int reg_coef;  // the kernel: 0 stream.cu, 2 stream2.cu or stream2m.cu, 3 stream64.cu,
+                 // 4 its kernel for short streams
   int packed;    // stream2.cu: fp32x2 arithmetic on pairs of mu cells
   int filled;    // stream2.cu: M fills the bin, m0 = M/2 (guards known at compile time)
   int npt;       // stream2.cu: list nodes per thread
@@ -93,7 +93,6 @@ int launch_seed_check32(const RunView &r, cudaStream_t st, uint64_t *launches);
 // node.cu -- AdiabaticFocusing + AdiabaticChange
 struct NodePlan {
   int pmax;        // register slots per thread (>= max(E, M); FP32 form: >= M)
-  int pcol;        // FP32 form: register slots of a change column (>= E)
   int threads;     // threads per CTA
   int nodes;       // nodes per CTA
   size_t smem;     // dynamic shared memory bytes

@@ -114,7 +114,6 @@ int plan_node32(int E, int M, size_t nodes, NodePlan *plan) {
     }
   }
   plan->pmax = bucket(M);
-  plan->pcol = E;
   return 0;
 }
 

@@ -30,31 +30,30 @@ namespace cg = cooperative_groups;
 namespace eprem {
 
 // Threads per CTA (multiples of 128, the register-allocation granule).
-template <typename Real, int MMAX, bool RegCoef> struct StreamShape;
-#define EPREM_STREAM_SHAPE(R, MM, RC, TT) \
-  template <> struct StreamShape<R, MM, RC> { static constexpr int T = TT; };
-EPREM_STREAM_SHAPE(double, 8, false, 1024)
-EPREM_STREAM_SHAPE(double, 16, false, 768)
-EPREM_STREAM_SHAPE(double, 24, false, 512)
-EPREM_STREAM_SHAPE(double, 32, false, 512)
-EPREM_STREAM_SHAPE(double, 40, false, 512)
-EPREM_STREAM_SHAPE(double, 48, false, 384)
-EPREM_STREAM_SHAPE(double, 64, false, 384)
+template <typename Real, int MMAX> struct StreamShape;
+#define EPREM_STREAM_SHAPE(R, MM, TT) \
+  template <> struct StreamShape<R, MM> { static constexpr int T = TT; };
+EPREM_STREAM_SHAPE(double, 8, 1024)
+EPREM_STREAM_SHAPE(double, 16, 768)
+EPREM_STREAM_SHAPE(double, 24, 512)
+EPREM_STREAM_SHAPE(double, 32, 512)
+EPREM_STREAM_SHAPE(double, 40, 512)
+EPREM_STREAM_SHAPE(double, 48, 384)
+EPREM_STREAM_SHAPE(double, 64, 384)
 #undef EPREM_STREAM_SHAPE
 
-// Shared memory of one CTA: coefficient table (shared-coefficient shapes) and
-// the halo slots.
-template <typename Real, int MMAX, bool RegCoef>
+// Shared memory of one CTA: coefficient table and the halo slots.
+template <typename Real, int MMAX>
 constexpr size_t stream_smem_bytes() {
-  constexpr int T = StreamShape<Real, MMAX, RegCoef>::T;
+  constexpr int T = StreamShape<Real, MMAX>::T;
   constexpr int W = T / 32;
-  return (RegCoef ? 0 : sizeof(Real) * MMAX * T) + sizeof(Real) * 2 * 2 * (W + 1) * MMAX;
+  return sizeof(Real) * MMAX * T + sizeof(Real) * 2 * 2 * (W + 1) * MMAX;
 }
 
-template <typename Real, int MMAX, bool RegCoef>
-__global__ void __launch_bounds__((StreamShape<Real, MMAX, RegCoef>::T), 1)
+template <typename Real, int MMAX>
+__global__ void __launch_bounds__((StreamShape<Real, MMAX>::T), 1)
     k_stream(RunView r, int m0) {
-  constexpr int T = StreamShape<Real, MMAX, RegCoef>::T;
+  constexpr int T = StreamShape<Real, MMAX>::T;
   constexpr int W = T / 32;
   constexpr unsigned FULL = 0xffffffffu;
   // halo slots, double-buffered by sub-cycle parity p:
@@ -63,8 +62,8 @@ __global__ void __launch_bounds__((StreamShape<Real, MMAX, RegCoef>::T), 1)
   //   lo[p][w][mu], w = 0..W : slot w holds lane 0 of warp w; slot W the next
   //                            CTA's first lane (written remotely).
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  Real *coef = reinterpret_cast<Real *>(sm_raw);  // [mu][T], shared-coefficient shapes
-  Real *halo = coef + (RegCoef ? 0 : MMAX * T);
+  Real *coef = reinterpret_cast<Real *>(sm_raw);  // [mu][T]
+  Real *halo = coef + MMAX * T;
   auto hi = [&](int p, int w) { return halo + ((p * 2 + 0) * (W + 1) + w) * MMAX; };
   auto lo = [&](int p, int w) { return halo + ((p * 2 + 1) * (W + 1) + w) * MMAX; };
 
@@ -98,12 +97,11 @@ __global__ void __launch_bounds__((StreamShape<Real, MMAX, RegCoef>::T), 1)
   const int i = crank * T + tid;
   const bool active = i < L;
   const size_t sN = (size_t)s * N;
-  Real fr[MMAX], cf[RegCoef ? MMAX : 1];
+  Real fr[MMAX];
 #pragma unroll
   for (int mu = 0; mu < MMAX; ++mu) {
     fr[mu] = (Real)0;
-    if (RegCoef) cf[mu] = (Real)0;
-    else if (mu < M) coef[mu * T + tid] = (Real)0;
+    if (mu < M) coef[mu * T + tid] = (Real)0;
   }
   double emt = 0.0;
   Real bcv = (Real)0;
@@ -130,10 +128,7 @@ __global__ void __launch_bounds__((StreamShape<Real, MMAX, RegCoef>::T), 1)
         const bool edge_cell = (mu >= m0) ? (i == 0) : (i == L - 1);
         const double del_fac = ec.vgrid * dtProp * r.mugrid[mu];
         const Real c = edge_cell ? (Real)0 : (Real)(mult * del_fac);
-        if (RegCoef)
-          cf[mu] = c;
-        else
-          coef[mu * T + tid] = c;
+        coef[mu * T + tid] = c;
       }
     }
     if (r.use_bc && i < 3) {
@@ -190,7 +185,7 @@ __global__ void __launch_bounds__((StreamShape<Real, MMAX, RegCoef>::T), 1)
 #pragma unroll
     for (int mu = 0; mu < MMAX; ++mu) {
       if (mu < M) {
-        const Real c = RegCoef ? cf[mu] : coef[mu * T + tid];
+        const Real c = coef[mu * T + tid];
         Real fn;
         if (mu >= m0) {  // mugrid[mu] >= 0: upwind from list node i-1
           Real nb = __shfl_up_sync(FULL, fr[mu], 1);
@@ -252,16 +247,16 @@ __global__ void k_seed_check(RunView r) {
 
 static const int kStreamBins[] = {8, 16, 24, 32, 40, 48, 64};
 
-template <typename Real, bool RC>
+template <typename Real>
 static int threads_for(int mmax) {
   switch (mmax) {
-    case 8: return StreamShape<Real, 8, RC>::T;
-    case 16: return StreamShape<Real, 16, RC>::T;
-    case 24: return StreamShape<Real, 24, RC>::T;
-    case 32: return StreamShape<Real, 32, RC>::T;
-    case 40: return StreamShape<Real, 40, RC>::T;
-    case 48: return StreamShape<Real, 48, RC>::T;
-    default: return StreamShape<Real, 64, RC>::T;
+    case 8: return StreamShape<Real, 8>::T;
+    case 16: return StreamShape<Real, 16>::T;
+    case 24: return StreamShape<Real, 24>::T;
+    case 32: return StreamShape<Real, 32>::T;
+    case 40: return StreamShape<Real, 40>::T;
+    case 48: return StreamShape<Real, 48>::T;
+    default: return StreamShape<Real, 64>::T;
   }
 }
 
@@ -319,17 +314,17 @@ int plan_stream(int precision, int N, int M, int m0, int variant, bool mirror_ok
   plan->mmax = mmax;
   plan->reg_coef = 0;
   plan->mirror = 0;
-  plan->threads = threads_for<double, false>(mmax);
+  plan->threads = threads_for<double>(mmax);
   plan->cluster = (N + plan->threads - 1) / plan->threads;
   if (plan->cluster > 8) return EPREM_GPU_ERR_ARG;  // portable cluster limit
   return 0;
 }
 
-template <typename Real, int MMAX, bool RC>
+template <typename Real, int MMAX>
 static cudaError_t launch_stream_t(const RunView &r, int cluster, int m0, cudaStream_t st) {
-  constexpr int T = StreamShape<Real, MMAX, RC>::T;
-  constexpr size_t dyn = stream_smem_bytes<Real, MMAX, RC>();
-  auto kern = k_stream<Real, MMAX, RC>;
+  constexpr int T = StreamShape<Real, MMAX>::T;
+  constexpr size_t dyn = stream_smem_bytes<Real, MMAX>();
+  auto kern = k_stream<Real, MMAX>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
   if (e != cudaSuccess) return e;
@@ -348,17 +343,17 @@ static cudaError_t launch_stream_t(const RunView &r, int cluster, int m0, cudaSt
   return cudaLaunchKernelEx(&cfg, kern, r, m0);
 }
 
-template <typename Real, bool RC>
+template <typename Real>
 static cudaError_t dispatch_mmax(const RunView &r, const StreamPlan &pl, int m0,
                                  cudaStream_t st) {
   switch (pl.mmax) {
-    case 8: return launch_stream_t<Real, 8, RC>(r, pl.cluster, m0, st);
-    case 16: return launch_stream_t<Real, 16, RC>(r, pl.cluster, m0, st);
-    case 24: return launch_stream_t<Real, 24, RC>(r, pl.cluster, m0, st);
-    case 32: return launch_stream_t<Real, 32, RC>(r, pl.cluster, m0, st);
-    case 40: return launch_stream_t<Real, 40, RC>(r, pl.cluster, m0, st);
-    case 48: return launch_stream_t<Real, 48, RC>(r, pl.cluster, m0, st);
-    default: return launch_stream_t<Real, 64, RC>(r, pl.cluster, m0, st);
+    case 8: return launch_stream_t<Real, 8>(r, pl.cluster, m0, st);
+    case 16: return launch_stream_t<Real, 16>(r, pl.cluster, m0, st);
+    case 24: return launch_stream_t<Real, 24>(r, pl.cluster, m0, st);
+    case 32: return launch_stream_t<Real, 32>(r, pl.cluster, m0, st);
+    case 40: return launch_stream_t<Real, 40>(r, pl.cluster, m0, st);
+    case 48: return launch_stream_t<Real, 48>(r, pl.cluster, m0, st);
+    default: return launch_stream_t<Real, 64>(r, pl.cluster, m0, st);
   }
 }
 
@@ -367,7 +362,7 @@ int launch_stream(const RunView &r, const StreamPlan &plan, int m0, cudaStream_t
   if (plan.reg_coef == 2) return launch_stream2(r, plan, m0, st, launches);
   if (r.precision != EPREM_FP64) return EPREM_GPU_ERR_ARG;
   if (plan.reg_coef >= 3) return launch_stream64(r, plan, m0, st, launches);
-  const cudaError_t err = dispatch_mmax<double, false>(r, plan, m0, st);
+  const cudaError_t err = dispatch_mmax<double>(r, plan, m0, st);
   *launches += 1;
   return err == cudaSuccess ? 0 : EPREM_GPU_ERR_CUDA;
 }
