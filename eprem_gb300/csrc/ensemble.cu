@@ -98,6 +98,7 @@ int tune_stream(eprem_gpu_run *r, int *chosen) {
   if (best_variant) {
     r->splan = best_plan;
     r->params.stream_variant = best_variant;
+    r->named_shape = false;
   }
   *chosen = r->params.stream_variant;
   return EPREM_GPU_OK;
@@ -158,6 +159,7 @@ extern "C" int eprem_gpu_set_stream_variant(eprem_gpu_run *r, int variant) {
     return fail(EPREM_GPU_ERR_ARG, "streaming variant does not fit this run's sizes");
   r->splan = pl;
   r->params.stream_variant = variant;
+  r->named_shape = variant / 8 != 0;
   return EPREM_GPU_OK;
 }
 
@@ -293,6 +295,7 @@ extern "C" int eprem_gpu_ensemble_autotune(eprem_gpu_ensemble *e, int *chosen_va
     } else {
       rc = eprem_gpu_set_stream_variant(r, variant);
       if (rc) return rc;
+      r->named_shape = false;
     }
     if (chosen_variants) chosen_variants[i] = variant;
   }
@@ -347,13 +350,16 @@ static int ensemble_capture_lockstep(eprem_gpu_ensemble *e) {
   std::vector<S2Group> groups;
   std::vector<int> solo;
   // runs of one size share a launch: the automatic shape is chosen for all
-  // their slabs (a slab's values do not depend on the shape)
+  // their slabs (a slab's values do not depend on the shape), also where the
+  // autotuner, which times a run alone, gave the mirrored kernel another width (16
+  // runs of 24 x 400 x 20 x 20: 36.8 ms a step with that width, 31.3 with the merged
+  // launch's); a shape that the caller named stays
   auto merged_plan = [&](eprem_gpu_run *r) {
     StreamPlan pl = r->splan;
-    if (!pl.mirror || r->params.stream_variant / 8) return pl;
+    if (!pl.mirror || r->named_shape) return pl;
     long long slabs = 0;
     for (eprem_gpu_run *o : e->runs)
-      if (o->splan.mirror && !(o->params.stream_variant / 8) && o->dims.num_mu == r->dims.num_mu &&
+      if (o->splan.mirror && !o->named_shape && o->dims.num_mu == r->dims.num_mu &&
           o->dims.num_nodes == r->dims.num_nodes)
         slabs += o->slabs();
     plan_stream2m(r->dims.num_nodes, r->dims.num_mu, r->m0, true, 0, slabs, &pl);

@@ -162,6 +162,7 @@ extern "C" int eprem_gpu_create(const eprem_dims_t *dims, const eprem_params_t *
   r->mirror_ok = dims->precision == EPREM_FP64 ? mirror64 : bc && even_mu;
   int prc = plan_stream(dims->precision, N, M, m0, params->stream_variant,
                         r->mirror_ok, (long long)S * E, &r->splan);
+  r->named_shape = params->stream_variant / 8 != 0;
   const bool fast64 = dims->precision == EPREM_FP64 && params->adiabatic_focus_alg <= 2 &&
                       params->adiabatic_change_alg <= 2;
   if (!prc)

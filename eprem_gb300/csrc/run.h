@@ -34,6 +34,7 @@ struct eprem_gpu_run {
   eprem::RunView v{};
   eprem::MhdParams mhd{};
   eprem::StreamPlan splan{};
+  bool named_shape = false;  // its shape was named by the caller (not by the autotuner)
   std::string skernel;  // eprem_gpu_stream_kernel's text
   eprem::NodePlan nplan{};
   int m0 = 0;
