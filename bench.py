@@ -48,9 +48,9 @@ BYTES_PER_CELL_UPDATE = {"fp64": 32.0, "fp32": 16.0}
 # traffic per launch / 96*1000*50*40 cells; traffic grows with the number of
 # (stream, energy) slabs, so it scales to a full launch by the cells processed.
 NCU_DRAM_BYTES_PER_CELL = {("stream", "fp32"): 1599.6e6 / 192e6,
-                           ("stream", "fp64"): 3055.1e6 / 192e6,
+                           ("stream", "fp64"): 3047.9e6 / 192e6,
                            ("node", "fp32"): 1501.7e6 / 192e6,
-                           ("node", "fp64"): 3024.5e6 / 192e6}
+                           ("node", "fp64"): 3024.1e6 / 192e6}
 
 
 # ---------------------------------------------------------------------------

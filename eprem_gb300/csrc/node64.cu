@@ -18,10 +18,10 @@
 // A CTA holds G whole nodes in shared memory; focusing takes a (node, energy)
 // row per thread, change a (node, mu) column, rows at an odd pitch (no bank
 // conflicts either way).
-// Per launch on a GB300 (node.cu before; with CUDA's log and exp between): 6 x
-// 1000 x 50 x 40, 3.71 -> 1.45 -> 0.93 ms (48 FP64 slots a cell); 24 x 400 x 20 x
-// 20, 1.33 -> 0.40 -> 0.24 ms; third order, 24 x 200 x 20 x 20, 1.80 -> 0.60 ->
-// 0.52 ms.
+// Per launch on a GB300 (node.cu before): 6 x 1000 x 50 x 40, 3.71 -> 1.17 ms (0.93
+// with two operations a cell in Euler passes); 24 x 400 x 20 x 20, 1.33 -> 0.29 ms
+// (0.24); third order, 24 x 200 x 20 x 20, 1.80 -> 0.46 ms.  CUDA's log and exp took
+// 0.52 ms more at 6 x 1000 x 50 x 40.
 #include "common.cuh"
 #include "kernels.h"
 #include "math64.cuh"

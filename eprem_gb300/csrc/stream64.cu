@@ -21,8 +21,8 @@
 // What that costs in precision is made good every kAnew sub-cycles:
 //   * b keeps an error of the last place of the largest value that it had, so it
 //     is formed anew from the cells: a node that drains by decades (weak
-//     scattering, a pulse that has passed) would otherwise end with it (5e-9 of f
-//     after 13,000 sub-cycles behind a pulse of 1e15).
+//     scattering, a pulse that has passed) would otherwise end with it (1e-8 of f
+//     after 11,000 sub-cycles behind a pulse of 1e15; 2e-14 now).
 //   * for a node's particle number to be kept over 1e5 sub-cycles A_j + C_j must be
 //     em exactly, so C_j is a multiple of em's last place, which makes the
 //     difference exact.  Rounded once for all it would move f at a speed that is
@@ -45,15 +45,16 @@
 //
 // Measured on a GB300, per launch, against the four-operation kernel of
 // stream.cu with its fixed CTA widths: 6 streams x 1000 x 50 x 40, 17.9 ->
-// 12.3 ms (two CTAs of 512 threads per slab; 85 % of the FP64 FMA peak; with
-// {A, C} per cell instead, four CTAs of 256 threads, 13.9 ms: clusters of four
-// leave 8 of the 152 SMs without work, and 8 warps do not cover the loads);
-// 24 x 400 x 20 x 20, 1.53 -> 0.90 ms (13 warps, so one scheduler of an SM has
-// four of them and the others three: the rest of the peak); 24 x 60 x 12 x 6
-// with 13,000 sub-cycles, 12.9 -> 0.91 ms (k_stream64_short on 128 threads where
-// the fixed width was 1024; latency of the chain of one sub-cycle).  The FP64 pipe takes a warp's
-// FMA in 64 cycles of its scheduler however independent, an addition or a
-// product alone in 76.
+// 12.6 ms (two CTAs of 512 threads per slab; the FP64 pipe 92 % busy at 96 such
+// streams; 12.1 without the sums and roundings anew; with {A, C} per cell instead,
+// four CTAs of 256 threads, 13.9 ms: clusters of four leave 8 of the 152 SMs
+// without work, and 8 warps do not cover the loads); 24 x 400 x 20 x 20, 1.53 ->
+// 0.92 ms (13 warps, so one scheduler of an SM has four of them and the others
+// three: the rest of the peak); 24 x 60 x 12 x 6 with 13,000 sub-cycles, 12.9 ->
+// 0.99 ms (k_stream64_short on 128 threads where the fixed width was 1024; latency
+// of the chain of one sub-cycle; 0.91 without the sums and roundings).  The FP64
+// pipe takes a warp's FMA in 64 cycles of its scheduler however independent, an
+// addition or a product alone in 76.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -337,7 +338,8 @@ __global__ void __launch_bounds__(TMAX, 1) k_stream64(RunView r, int m0) {
 // at 64 cycles each there, so the directions of mu go to a thread each, which has
 // half of them (both form b, from the moments in shared memory: 6 H + 6
 // operations per node where the other kernel takes 6 H + 2).  24 streams x 60 x
-// 12 x 6 with 13,000 sub-cycles, per launch: 1.44 -> 0.91 ms.
+// 12 x 6 with 13,000 sub-cycles, per launch: 1.44 -> 0.91 ms, 0.99 with the sums
+// and roundings anew.
 template <int H, int HLO>
 __global__ void __launch_bounds__(2 * kS64ShortNodes, 1) k_stream64_short(RunView r, int m0) {
   constexpr unsigned FULL = 0xffffffffu;
@@ -527,7 +529,8 @@ __global__ void __launch_bounds__(2 * kS64ShortNodes, 1) k_stream64_short(RunVie
 // cells or a portable cluster (8 CTAs) cannot hold the stream; those runs keep
 // the kernel of stream.cu, which takes any mu grid and longer streams.
 // The short streams' kernel, by the warps per SM that a launch of the other one
-// would have (12 energies, 10 sub-steps, ms of the other one and of this one): M
+// would have (12 energies, 10 sub-steps, ms of the other one and of this one,
+// before either formed sums and roundings anew): M
 // = 6, N = 64, 3.8 warps 0.56 and 0.44, 8.5 0.68 and 0.68, 15 0.86 and 0.95; M =
 // 20, N = 128, 1.9 2.88 and 2.44, 17 4.64 and 4.12, 30 6.5 and 6.6; M = 40, N =
 // 64, 3.8 2.83 and 1.78, 15 4.28 and 3.71; N = 96, 23 7.69 and 7.79.
